@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "gpurir_internal.cuh"
+#include "ism_moment.cuh"
 #include "../../include/gpurir_gb300.h"
 
 namespace gpurir {
@@ -426,6 +427,11 @@ struct Plan {
     int mode = 0, tw = 0;   // tap evaluation mode (0 FP32, 1 mixed precision, 2 LUT), window length
     int max_n_diff;
     bool skip_flags = false;   // some segment starts past the rooms' delay bound: test items on the device
+    // fractional-delay moment path (ism_moment.cu); nullptr: taps one by one (ism_forward.cu)
+    const MomBasis *mom = nullptr;
+    int mom_T = 0;                // longest segment
+    int mom_win = 0;              // shortest last segment of an item
+    size_t mom_smem = 0;
     std::vector<IsmItem> items;
     std::vector<IsmItem> rirs;
 };
@@ -463,8 +469,9 @@ static double room_span(const RoomDesc &r) {
 // what one block's shared memory holds; RIRs of small launches are cut finer so
 // that the persistent grid has work for every SM.  Items are ordered by an
 // estimate of their cost, largest first (longest-processing-time order).
-static int plan_rooms(gpurir_sim *s, const std::vector<RoomDesc> &R, Plan &P) {
+static int plan_taps(gpurir_sim *s, const std::vector<RoomDesc> &R, Plan &P) {
     int max_nsub = 0;
+    P.mom = nullptr;
     P.mode = s->lut ? 2 : (s->mp ? 1 : 0);
     if (P.mode != 0 && s->comp > 0) {   // compensated accumulation (mode flag 4, ism_forward.cu)
         int longest = 0;
@@ -594,6 +601,186 @@ static int plan_rooms(gpurir_sim *s, const std::vector<RoomDesc> &R, Plan &P) {
     return GPURIR_OK;
 }
 
+// Images of a room with a delay in [a, b) samples: the mirrored rooms fill space with
+// one image each, cut off by the image grid.
+static double shell_images(const RoomDesc &r, double a, double b) {
+    const double k = (double)r.kh + r.kl, v = (double)r.L[0] * r.L[1] * r.L[2];
+    auto ball = [&](double t) {
+        const double d = std::max(t, 0.0) / k;
+        double grid = 1.0;   // the same ball's bounding box, cut off by the grid
+        for (int e = 0; e < 3; e++) grid *= std::min<double>(r.nb[e], 2.0 * d / r.L[e] + 1.0);
+        return std::min(4.1887902 * d * d * d / v + 1.0, grid);
+    };
+    return std::max(ball(b) - ball(a), 0.0);
+}
+
+// Work items of the moment path: segments of at most T samples, the last one of an RIR
+// long enough to hold its envelope window (so that its item writes the diffuse tail), and
+// in launches of few RIRs the image rows of heavy segments dealt to several items whose
+// partial segments are added up afterwards.
+static int plan_moment(gpurir_sim *s, const std::vector<RoomDesc> &R, Plan &P) {
+    P.mode = 0;
+    P.tw = (int)std::lround(2.0 * R[0].H);
+    P.mom = &moment_basis_cached(P.tw);
+    P.items.clear();
+    P.rirs.clear();
+    P.groups.clear();
+    P.skip_flags = false;
+    P.part_floats = 0;
+    P.max_part_len = 0;
+    P.unfused_tails = 0;
+    P.max_n_diff = 0;
+    P.axis_cap = 0;
+    long M_tot = 0;
+    double covered = 0.0;   // samples of all early parts that an image can reach
+    for (const RoomDesc &r : R) {
+        M_tot += (long)r.n_src * r.n_rcv;
+        P.max_n_diff = std::max(P.max_n_diff, r.n_total - r.n_ism);
+        P.axis_cap = std::max(P.axis_cap, r.nb[0] + r.nb[1] + r.nb[2]);
+        covered += (double)r.n_src * r.n_rcv * std::min<double>(r.n_ism, room_span(r));
+    }
+    // Costs in cycles of one SM with two blocks at work (measured): 2.9 per image (the
+    // integer atomics of 32 images take ~90), and per segment the filter, the sums' zeroing
+    // and their way into the basis, ~8000 at 1024 samples and 16 kHz.
+    const double per_image = 2.9;
+    auto segment_cost = [&](int T) { return 0.11 * T * P.mom->n_quads + 3000.0; };
+    double images = 0.0;
+    for (const RoomDesc &r : R)
+        images += (double)r.n_src * r.n_rcv * shell_images(r, 0.0, std::min<double>(r.n_ism, room_span(r)));
+    // Long segments spend less on what neighbours share (their taps' reach, 12 % of the images at
+    // 1024 samples and 16 kHz, 25 % at 512); short ones give a small launch more items.  A
+    // segment of many images can be dealt to several items instead.
+    const long slots = 2L * s->num_sms;   // (not of a tuned grid: the items fix the results' bits)
+    P.mom_T = 1024;
+    if (covered / 1024 < slots && images * per_image < 2.0 * covered / 1024 * segment_cost(1024)) P.mom_T = 512;
+    if (moment_cells(P.mom_T, *P.mom) > kMomCells || moment_smem_bytes(P.mom_T, P.axis_cap, *P.mom) > kSmemBudget)
+        P.mom_T = 512;   // (long windows: two blocks per SM)
+    P.mom_smem = moment_smem_bytes(P.mom_T, P.axis_cap, *P.mom);
+    int bps = moment_blocks_per_sm(P.mom_smem);
+    if (bps < 1) return fail(GPURIR_ERR_CUDA, "ISM kernel does not fit on an SM");
+    if (tuning(1) > 0) bps = std::min(bps, tuning(1));   // ism_blocks_per_sm (tuning.cu)
+    const int T = P.mom_T;
+    const int win = (int)std::ceil(0.01 * R[0].fs) + 2;
+    P.mom_win = win <= T - 4 ? win : 0;
+    const double fixed = segment_cost(T);
+    struct Seg { int lo, hi; double cost; };
+    std::vector<std::vector<Seg>> segs(R.size());
+    double total = 0.0, images_cost = 0.0;
+    long busy = 0;   // segments with images
+    for (size_t ri = 0; ri < R.size(); ri++) {
+        const RoomDesc &r = R[ri];
+        const double span = room_span(r), M = (double)r.n_src * r.n_rcv;
+        for (int a = 0, b; a < r.n_ism; a = b) {   // as the kernel cuts an item's samples
+            b = std::min(a + T, r.n_ism);
+            if (b < r.n_ism && r.n_ism - b < P.mom_win) b = (r.n_ism - P.mom_win) & ~3;
+            Seg g = {a, b, 500.0};
+            if (a < span) {
+                const double c = per_image * shell_images(r, a - r.H, b + r.H);
+                g.cost += fixed + c;
+                images_cost += c * M;
+                busy += (long)M;
+            }
+            total += g.cost * M;
+            segs[ri].push_back(g);
+        }
+    }
+    // Parts.  Every part of a segment repeats its fixed cost, so a launch that does not fill
+    // the GPU is dealt out to one wave of blocks by images, and in a larger one only segments
+    // of twice a block's share are cut.  Light neighbours go into one item.
+    const double share = total / slots, image_share = images_cost / slots, most = total / (4.0 * slots);
+    P.rirs.reserve(M_tot);
+    std::vector<IsmItem> work;
+    std::vector<std::pair<double, int>> cost;
+    for (size_t ri = 0; ri < R.size(); ri++) {
+        const RoomDesc &r = R[ri];
+        const long M = (long)r.n_src * r.n_rcv;
+        // items of one RIR: a heavy segment as several interleaved parts, light ones in runs
+        struct Group { int lo, hi, parts; double cost; };
+        std::vector<Group> items;
+        for (const Seg &g : segs[ri]) {
+            const double images_of = std::max(g.cost - fixed - 500.0, 0.0);
+            double n = busy < slots ? std::floor(images_of / image_share) : (g.cost > 2.0 * share ? std::ceil(g.cost / share) : 1.0);
+            const int parts = (int)std::max(1.0, std::min(n, images_of / (per_image * 1024)));
+            if (!items.empty() && parts == 1 && items.back().parts == 1 && items.back().cost + g.cost <= most &&
+                (g.lo - items.back().lo) % T == 0) {
+                items.back().hi = g.hi;
+                items.back().cost += g.cost;
+            } else {
+                items.push_back({g.lo, g.hi, parts, g.cost});
+            }
+        }
+        const int last = items.empty() ? 0 : segs[ri].back().hi - segs[ri].back().lo;
+        const bool fused = !items.empty() && items.back().parts == 1 && r.n_total > r.n_ism &&
+                           (segs[ri].size() == 1 || last >= win);
+        for (long m = 0; m < M; m++) {
+            IsmItem it{};
+            it.room = (int)ri;
+            it.src = r.src_off + (int)(m / r.n_rcv);
+            it.rcv = r.rcv_off + (int)(m % r.n_rcv);
+            it.rir = r.rir_off + (int)m;
+            it.out_row = r.out_off + (long long)m * r.n_total;
+            IsmItem ref = it;
+            ref.t_hi = fused ? -1 : 0;   // -1: the tail kernel skips this RIR
+            P.rirs.push_back(ref);
+            if (!fused && r.n_total > r.n_ism) P.unfused_tails++;
+            for (const Group &g : items) {
+                IsmItem w = it;
+                w.t_lo = g.lo;
+                w.t_hi = g.hi;
+                w.part_off = -1;
+                w.i_hi = g.parts;
+                const int len = g.hi - g.lo;
+                if (g.parts > 1) {
+                    P.groups.push_back({it.out_row + g.lo, P.part_floats, len, g.parts});
+                    P.max_part_len = std::max(P.max_part_len, len);
+                }
+                for (int p = 0; p < g.parts; p++) {
+                    w.i_lo = p;
+                    if (g.parts > 1) {
+                        w.part_off = P.part_floats;
+                        P.part_floats += len;
+                    }
+                    cost.push_back({g.cost / g.parts, (int)work.size()});
+                    work.push_back(w);
+                }
+            }
+        }
+    }
+    std::stable_sort(cost.begin(), cost.end(), [](const std::pair<double, int> &x, const std::pair<double, int> &y) {
+        return x.first > y.first;
+    });
+    P.items.reserve(work.size());
+    for (auto &c : cost) P.items.push_back(work[c.second]);
+    P.grid = (int)std::min<long>((long)P.items.size(), (long)s->num_sms * bps);
+    return GPURIR_OK;
+}
+
+// Which kernel evaluates a launch.  The moment kernel serves the default FP32 mode at window
+// lengths from 48 (6 kHz; below, the window's ends inside a cell cost accuracy) to 400
+// samples (50 kHz; its cells' sums and filter fill two blocks per SM there), when the RIRs
+// have images enough: a sample's filter costs what the taps of some tenths of an image do,
+// and an RIR of few images is nearer to the FP64 sum with the taps (a single image: 3e-8
+// against 9e-8).  The line is a mean of 2048 images in reach per RIR at a window of 128
+// samples, fewer for longer windows: measured over 150 launches of 1 to 800 RIRs, 1 to 400000
+// images each, 6 to 48 kHz, the moment kernel takes 0.21-0.5 of the tap kernel's time on dense
+// rooms, 0.5-0.8 at 3000 to 10000 images, 0.75-1.05 below 2000.
+static bool use_moments(const gpurir_sim *s, const std::vector<RoomDesc> &R) {
+    const int tw = (int)std::lround(2.0 * R[0].H);
+    if (s->lut || s->mp || tw < kMomMinTw || tw > kMomMaxTw) return false;
+    double images = 0.0, rirs = 0.0;
+    for (const RoomDesc &r : R) {
+        if (r.n_ism > 3000000) return false;   // (cell indices are formed in FP32)
+        const double M = (double)r.n_src * r.n_rcv;
+        images += M * shell_images(r, 0.0, r.n_ism + r.H);
+        rirs += M;
+    }
+    return images * tw >= 2048.0 * 128.0 * rirs;
+}
+
+static int plan_rooms(gpurir_sim *s, const std::vector<RoomDesc> &R, Plan &P) {
+    return use_moments(s, R) ? plan_moment(s, R, P) : plan_taps(s, R, P);
+}
+
 static int check_status(gpurir_sim *s) {
     if (s->h_ctl[1] != 0) {
         int code = s->h_ctl[1];
@@ -605,7 +792,7 @@ static int check_status(gpurir_sim *s) {
 
 // Byte layout of one launch's descriptors (mirrored host staging -> device).
 struct Layout {
-    size_t o_rooms, o_items, o_rirs, o_groups, o_pos, o_pre, stage_bytes, o_env, o_axis, o_part, o_skip, o_out,
+    size_t o_rooms, o_items, o_rirs, o_groups, o_coef, o_pos, o_pre, stage_bytes, o_env, o_axis, o_part, o_skip, o_out,
         dev_bytes;
 };
 
@@ -620,10 +807,12 @@ static Layout make_layout(const Plan &P, size_t n_rooms, long n_src, long n_rcv,
     L.o_items = align_up(L.o_pre + (host_io ? (size_t)M : 0), 256);
     L.o_rirs = align_up(L.o_items + P.items.size() * sizeof(IsmItem), 256);
     L.o_groups = align_up(L.o_rirs + P.rirs.size() * sizeof(IsmItem), 256);
-    L.stage_bytes = align_up(L.o_groups + P.groups.size() * sizeof(PartGroup), 256);
+    L.o_coef = align_up(L.o_groups + P.groups.size() * sizeof(PartGroup), 256);   // filter of the moment path
+    L.stage_bytes = align_up(L.o_coef + (P.mom ? P.mom->coef.size() * sizeof(float2) : 0), 256);
     L.o_env = L.stage_bytes;
     L.o_axis = align_up(L.o_env + (size_t)M * 3 * sizeof(float), 256);
-    L.o_part = align_up(L.o_axis + (size_t)P.grid * P.axis_cap * sizeof(float4), 256);
+    // (the moment kernel holds the tables of two items per block)
+    L.o_part = align_up(L.o_axis + (size_t)P.grid * P.axis_cap * (P.mom ? 2 : 1) * sizeof(float4), 256);
     L.o_skip = align_up(L.o_part + (size_t)P.part_floats * sizeof(float), 256);
     L.o_out = align_up(L.o_skip + (P.skip_flags ? P.items.size() : 0), 256);
     L.dev_bytes = L.o_out + (host_io ? (size_t)out_elems * sizeof(float) : 0);
@@ -673,6 +862,7 @@ static void fill_stage(char *h, const Layout &L, const std::vector<RoomDesc> &R,
     if (!P.items.empty()) memcpy(h + L.o_items, P.items.data(), P.items.size() * sizeof(IsmItem));
     if (!P.rirs.empty()) memcpy(h + L.o_rirs, P.rirs.data(), P.rirs.size() * sizeof(IsmItem));
     if (!P.groups.empty()) memcpy(h + L.o_groups, P.groups.data(), P.groups.size() * sizeof(PartGroup));
+    if (P.mom) memcpy(h + L.o_coef, P.mom->coef.data(), P.mom->coef.size() * sizeof(float2));
 }
 
 // Enqueue the ISM and tail kernels of one planned launch on `st`.
@@ -701,7 +891,32 @@ static int enqueue_kernels(gpurir_sim *s, const Plan &P, const char *d, const La
             if (record) s->last_launches += 1;
         }
     }
-    if (P.grid > 0)
+    if (P.grid > 0 && P.mom) {
+        MomLaunch m{};
+        m.rooms = drooms;
+        m.items = reinterpret_cast<const IsmItem *>(d + L.o_items);
+        m.n_items = (int)P.items.size();
+        m.pos_src = dps; m.pos_rcv = dpr; m.orv_src = dos; m.orv_rcv = dor;
+        m.out = dout;
+        m.partial = reinterpret_cast<float *>(const_cast<char *>(d) + L.o_part);
+        m.work_counter = work_counter;
+        m.status = s->d_ctl + 1;
+        m.axis_tab = reinterpret_cast<float4 *>(const_cast<char *>(d) + L.o_axis);
+        m.axis_cap = P.axis_cap;
+        m.T = P.mom_T;
+        m.nbp = moment_cells(P.mom_T, *P.mom);
+        m.win = P.mom_win;
+        m.lead = P.mom->lead;
+        m.taps = P.mom->taps;
+        m.quads = P.mom->quads;
+        m.coef = reinterpret_cast<const float2 *>(d + L.o_coef);
+        memcpy(m.run, P.mom->run, sizeof(m.run));
+        m.n_quads = P.mom->n_quads;
+        memcpy(m.S, P.mom->S, sizeof(m.S));
+        m.seed = ta.seed; m.offset = ta.offset; m.offset_ptr = ta.offset_ptr;
+        m.noise_kind = ta.noise_kind; m.env_out = ta.env_out; m.fuse_tail = ta.fuse; m.tail_pre = ta.pre;
+        CK(moment_launch(m, P.mom_smem, P.grid, st));
+    } else if (P.grid > 0)
         CK(ism_forward_launch(P.tpl, drooms, reinterpret_cast<const IsmItem *>(d + L.o_items),
                               (int)P.items.size(), dps, dpr, dos, dor, dout, work_counter,
                               s->d_ctl + 1, P.em, P.nsub, P.clamp, P.grid, st, P.mode, P.tw, &ta,
@@ -1336,7 +1551,7 @@ static int backward_batch(gpurir_sim *s, int n_rooms, const gpurir_room *rooms, 
         if ((R[i].spkr != 0 && !d_orV_src) || (R[i].mic != 0 && !d_orV_rcv))
             return fail(GPURIR_ERR_INVALID, "orientation required for a non-omni pattern");
     Plan P;
-    if ((rc = plan_rooms(s, R, P))) return rc;
+    if ((rc = plan_taps(s, R, P))) return rc;
     int max_tseg = 1;
     for (const IsmItem &it : P.items) max_tseg = std::max(max_tseg, it.t_hi - it.t_lo);
     const int pad = 64 * P.tpl;
@@ -1439,7 +1654,10 @@ extern "C" int gpurir_adjoint_create(gpurir_sim *s, int n_rooms, const gpurir_ro
     a->n_rooms = n_rooms;
     std::vector<RoomDesc> R;
     int rc = build_batch(n_rooms, rooms, Fs, c, R, a->ns, a->nr, a->out_elems);
-    if (rc == GPURIR_OK) rc = plan_rooms(s, R, a->P);
+    // The differentiable forward keeps the taps, whose bits the gradients of positions follow:
+    // those are sums of large opposite terms, and another rounding of the RIRs (1e-7) moves
+    // them by up to 1e-4.
+    if (rc == GPURIR_OK) rc = plan_taps(s, R, a->P);
     if (rc) { delete a; return rc; }
     for (const RoomDesc &r : R) {
         a->need_orv_src |= r.spkr != 0;
