@@ -64,6 +64,15 @@ int traj_adjoint_grid(int M, int P, int num_sms);
 cudaError_t traj_adjoint_launch(const double *g, long n_out, const int *w_ini, const int *w_len, const float *rir,
                                 int P, int R, int L, int M, const float2 *W, const float2 *Sg, float *gt,
                                 float *grad_rir, float *grad_sig, float2 *acc, int grid, cudaStream_t st);
+struct BlkPlan {
+    int B, n_pair, runs, run_pairs, grid;
+};
+bool traj_adjoint_blk_plan(int P, int R, int L, int S, int num_sms, BlkPlan &b);
+size_t traj_adjoint_blk_floats(const BlkPlan &b, int P, int S);
+int traj_adjoint_blk_fft();
+cudaError_t traj_adjoint_blk_launch(const double *g, long n_out, const int *w_ini, const int *w_len, const float *seg,
+                                    const float *rir, int P, int R, int L, int S, const BlkPlan &b, const float2 *W,
+                                    float *gt, float *work, float *grad_rir, float *grad_sig, cudaStream_t st);
 cudaError_t room_beta_launch(RoomDesc *rooms, int n_rooms, const float *beta, cudaStream_t st);
 int l2_grad_blocks(long n);
 int tuning(int knob);
@@ -1993,15 +2002,19 @@ extern "C" int gpurir_trajectory_adjoint_device(gpurir_sim *s, const float *d_se
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     const long n = (long)seg_len + rir_len - 1;
     if (n > 16384) return fail(GPURIR_ERR_UNSUPPORTED, "trajectory adjoint: segment + RIR longer than 16384 samples");
-    // the register FFT kernels cover N = 2048 .. 16384: shorter problems are zero-padded to 2048
-    const int N = std::max(fft_size(n), 2048), M = N / 2;
     const long n_out = (long)w_ini[n_pts] + rir_len - 1;
+    // short segments: blocks of lags, one 2048-point problem each; else whole rows (the register
+    // FFT kernels cover N = 2048 .. 16384: shorter problems are zero-padded to 2048)
+    BlkPlan blk{};
+    const bool blocks = traj_adjoint_blk_plan(n_pts, n_rcv, rir_len, seg_len, s->num_sms, blk);
+    const int N = blocks ? traj_adjoint_blk_fft() : std::max(fft_size(n), 2048), M = N / 2;
     const int grid = traj_adjoint_grid(M, n_pts, s->num_sms);
     if (s->conv_recorded) CK(cudaStreamWaitEvent(st, s->conv_busy, 0));
-    const size_t o_sg = 0;
-    const size_t o_gt = align_up(o_sg + (size_t)n_pts * (M + 1) * sizeof(float2), 256);
-    const size_t o_acc = align_up(o_gt + (size_t)n_rcv * n_out * sizeof(float), 256);
-    const size_t o_win = align_up(o_acc + (size_t)grid * (M + 1) * sizeof(float2), 256);
+    const size_t o_sg = 0;   // spectra and partial sums, or spectra and accumulators
+    const size_t o_acc = align_up(o_sg + (size_t)n_pts * (M + 1) * sizeof(float2), 256);
+    const size_t o_gt = blocks ? align_up(traj_adjoint_blk_floats(blk, n_pts, seg_len) * sizeof(float), 256)
+                               : align_up(o_acc + (size_t)grid * (M + 1) * sizeof(float2), 256);
+    const size_t o_win = align_up(o_gt + (size_t)n_rcv * n_out * sizeof(float), 256);
     const size_t bytes = align_up(o_win + win.size() * sizeof(int), 256);
     if ((rc = ensure_conv(s, bytes))) return rc;
     const float2 *W = nullptr;
@@ -2012,11 +2025,17 @@ extern "C" int gpurir_trajectory_adjoint_device(gpurir_sim *s, const float *d_se
     CK(cudaMemcpyAsync(dwin, s->h_stage, win.size() * sizeof(int), cudaMemcpyHostToDevice, st));
     CK(cudaEventRecord(s->stage_done, st));
     s->stage_pending = true;
-    float2 *Sg = reinterpret_cast<float2 *>(s->d_conv + o_sg);
-    CK(segment_spectra_launch(d_segments, n_pts, seg_len, M, W, Sg, nullptr, s->num_sms, st));
-    CK(traj_adjoint_launch(d_grad_out, n_out, dwin, dwin + n_pts + 1, d_rir, n_pts, n_rcv, rir_len, M, W, Sg,
-                           reinterpret_cast<float *>(s->d_conv + o_gt), d_grad_rir, d_grad_signal,
-                           reinterpret_cast<float2 *>(s->d_conv + o_acc), grid, st));
+    float *gt = reinterpret_cast<float *>(s->d_conv + o_gt);
+    if (blocks) {
+        CK(traj_adjoint_blk_launch(d_grad_out, n_out, dwin, dwin + n_pts + 1, d_segments, d_rir, n_pts, n_rcv, rir_len,
+                                   seg_len, blk, W, gt, reinterpret_cast<float *>(s->d_conv + o_sg), d_grad_rir,
+                                   d_grad_signal, st));
+    } else {
+        float2 *Sg = reinterpret_cast<float2 *>(s->d_conv + o_sg);
+        CK(segment_spectra_launch(d_segments, n_pts, seg_len, M, W, Sg, nullptr, s->num_sms, st));
+        CK(traj_adjoint_launch(d_grad_out, n_out, dwin, dwin + n_pts + 1, d_rir, n_pts, n_rcv, rir_len, M, W, Sg, gt,
+                               d_grad_rir, d_grad_signal, reinterpret_cast<float2 *>(s->d_conv + o_acc), grid, st));
+    }
     CK(cudaEventRecord(s->conv_busy, st));
     s->conv_recorded = true;
     return GPURIR_OK;

@@ -947,6 +947,283 @@ __global__ void __launch_bounds__(M / 16) traj_adjoint_kernel(
     }
 }
 
+// ---------------------------------------------------------------------------
+// The adjoint in blocks of lags, for segments far shorter than the RIRs.
+//
+// traj_adjoint_kernel transforms whole rows: N = 16384 for the 400-sample segments and
+// 12800-sample RIRs of a trajectory, one 139 KB block per SM that waits for its row
+// loads (568 us for 3200 rows).  A correlation with a segment of S samples only needs
+// windows of S + B - 1 samples for B lags, so here the lags of a row are cut into blocks
+// of B <= 2049 - S and every block is one 2048-point problem:
+//   dL/dh[b B + k] = sum_t g[b B + k + t] x[t],   dL/dx[t] += sum_k g[b B + k + t] h[b B + k]
+// (no circular wrap: k + t <= 2047).  Two blocks go through one complex transform as real
+// and imaginary part: with G = G1 + i G2 and X the spectrum of the real x, the inverse of
+// G conj(X) is d1 + i d2, and the real part of the inverse of G conj(H) is the sum of both
+// blocks' parts of dL/dx -- no unpacking of real spectra at all.
+//
+// 128 threads, 16 values each: radix 16, 16, 8 forward and 8, 16, 16 back, so that a
+// thread's spectral bins j + 128 g + 256 s are the same for every transform and the
+// spectral step stays in registers.  Work item = a run of block pairs of one point; the
+// run's part of dL/dx goes to `part` and a second kernel adds the runs in order.
+//
+// Forward and adjoint of the 400-point workload (3200 rows of 12800 samples) took 930 us with
+// whole rows and take 608 us with blocks, the adjoint alone ~565 and ~240; 500 MB of rows
+// read and written are 75 us of that, the transforms' arithmetic the rest.
+constexpr int kBlk = 2048;                  // points of a block's transform
+constexpr int kBlkThreads = 128;
+constexpr int kBlkPerSm = 4;                // resident blocks (128 registers; at 96 and five blocks 1 % slower)
+constexpr int kBlkMaxSeg = 1024;            // longest segment served (half of a block for the lags)
+
+// DFT of eight values in place (outputs in order), as reg_fft's last pass.
+template <bool INV>
+__device__ __forceinline__ void dft8(float2 &a0, float2 &a1, float2 &a2, float2 &a3, float2 &a4, float2 &a5,
+                                     float2 &a6, float2 &a7) {
+    dft4<INV>(a0, a2, a4, a6);
+    dft4<INV>(a1, a3, a5, a7);
+    const float2 w1 = make_float2(kR2, INV ? kR2 : -kR2);
+    const float2 w3 = make_float2(-kR2, INV ? kR2 : -kR2);
+    const float2 o0 = a1, o1 = cmul(a3, w1), o2 = rot_q<INV>(a5), o3 = cmul(a7, w3);
+    const float2 e0 = a0, e1 = a2, e2 = a4, e3 = a6;
+    a0 = cadd(e0, o0); a4 = csub(e0, o0);
+    a1 = cadd(e1, o1); a5 = csub(e1, o1);
+    a2 = cadd(e2, o2); a6 = csub(e2, o2);
+    a3 = cadd(e3, o3); a7 = csub(e3, o3);
+}
+
+// Forward transform: v[r] = z[j + 128 r] in, v[8 g + s] = Z[j + 128 g + 256 s] out.
+// W: exp(-2 pi i m / 2048).
+__device__ __forceinline__ void blk_forward(float2 (&v)[16], float2 *buf, const float2 *__restrict__ W) {
+    constexpr int T = kBlkThreads;
+    const int j = threadIdx.x;
+    dft16<false>(v);
+    __syncthreads();   // buf is free
+#pragma unroll
+    for (int s = 0; s < 16; s++) buf[pad16(16 * j + s)] = v[dr16(s)];
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < 16; r++) v[r] = buf[pad16(j + r * T)];
+    const int k = j & 15;
+    {
+        float2 t[16];
+        twiddle_powers(W, k * (kBlk / 256), t);
+#pragma unroll
+        for (int r = 1; r < 16; r++) v[r] = cmul(v[r], t[r]);
+    }
+    dft16<false>(v);
+    __syncthreads();
+#pragma unroll
+    for (int s = 0; s < 16; s++) buf[pad16((j - k) * 16 + k + 16 * s)] = v[dr16(s)];
+    __syncthreads();
+#pragma unroll
+    for (int g = 0; g < 2; g++) {
+        const int jj = j + T * g;   // < 256
+        float2 *a = v + 8 * g;
+#pragma unroll
+        for (int r = 0; r < 8; r++) a[r] = buf[pad16(jj + 256 * r)];
+        const float2 t1 = __ldg(&W[jj]), t2 = __ldg(&W[2 * jj]), t4 = __ldg(&W[4 * jj]);
+        const float2 t3 = cmul(t1, t2);
+        a[1] = cmul(a[1], t1);
+        a[2] = cmul(a[2], t2);
+        a[3] = cmul(a[3], t3);
+        a[4] = cmul(a[4], t4);
+        a[5] = cmul(a[5], cmul(t1, t4));
+        a[6] = cmul(a[6], cmul(t2, t4));
+        a[7] = cmul(a[7], cmul(t3, t4));
+        dft8<false>(a[0], a[1], a[2], a[3], a[4], a[5], a[6], a[7]);
+    }
+}
+
+// Inverse transform (unnormalised): v[8 g + s] = Z[j + 128 g + 256 s] in, and out
+// v[dr16(s)] = z[j + 128 s].
+__device__ __forceinline__ void blk_inverse(float2 (&v)[16], float2 *buf, const float2 *__restrict__ W) {
+    constexpr int T = kBlkThreads;
+    const int j = threadIdx.x;
+#pragma unroll
+    for (int g = 0; g < 2; g++) {
+        float2 *a = v + 8 * g;
+        dft8<true>(a[0], a[1], a[2], a[3], a[4], a[5], a[6], a[7]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int g = 0; g < 2; g++)
+#pragma unroll
+        for (int s = 0; s < 8; s++) buf[pad16((j + T * g) * 8 + s)] = v[8 * g + s];
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < 16; r++) v[r] = buf[pad16(j + r * T)];
+    const int k = j & 7;
+    {
+        float2 t[16];
+        twiddle_powers(W, k * (kBlk / 128), t);
+#pragma unroll
+        for (int r = 1; r < 16; r++) v[r] = cmul(v[r], cconj(t[r]));
+    }
+    dft16<true>(v);
+    __syncthreads();
+#pragma unroll
+    for (int s = 0; s < 16; s++) buf[pad16((j - k) * 16 + k + 8 * s)] = v[dr16(s)];
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < 16; r++) v[r] = buf[pad16(j + r * T)];
+    {
+        float2 t[16];
+        twiddle_powers(W, j, t);
+#pragma unroll
+        for (int r = 1; r < 16; r++) v[r] = cmul(v[r], cconj(t[r]));
+    }
+    dft16<true>(v);
+}
+
+// Spectra of the segments as the block transforms hold them: X[p][n] conjugated, scaled by
+// 1 / 2048, in bin order.
+__global__ void __launch_bounds__(kBlkThreads) blk_spectra_kernel(const float *__restrict__ seg, int P, int S,
+                                                                  const float2 *__restrict__ W, float2 *__restrict__ X) {
+    __shared__ __align__(16) float2 buf[kBlk + kBlk / 16];
+    const int j = threadIdx.x;
+    for (int p = blockIdx.x; p < P; p += gridDim.x) {
+        float2 v[16];
+#pragma unroll
+        for (int r = 0; r < 16; r++) {
+            const int n = j + r * kBlkThreads;
+            v[r] = make_float2(n < S ? __ldg(&seg[(size_t)p * S + n]) : 0.0f, 0.0f);
+        }
+        blk_forward(v, buf, W);
+#pragma unroll
+        for (int i = 0; i < 16; i++)
+            X[(size_t)p * kBlk + j + kBlkThreads * (i >> 3) + 256 * (i & 7)] =
+                make_float2(v[i].x * (1.0f / kBlk), -v[i].y * (1.0f / kBlk));
+    }
+}
+
+// Pair u of a point: blocks 2 (u mod n_pair), + 1 of receiver u / n_pair.  (Both of one row, so
+// that a NaN or an infinity in one receiver's gradient stays out of the others' RIRs.)
+__global__ void __launch_bounds__(kBlkThreads, kBlkPerSm) traj_adjoint_blk_kernel(
+        const float *__restrict__ gt, long n_out, const int *__restrict__ w_ini, const int *__restrict__ w_len,
+        const float *__restrict__ rir, int P, int R, int L, int S, int B, int n_pair, int runs, int run_pairs,
+        const float2 *__restrict__ W, const float2 *__restrict__ X, float *__restrict__ grad_rir,
+        float *__restrict__ part) {
+    __shared__ __align__(16) float2 buf[kBlk + kBlk / 16];
+    __shared__ float2 acc[kBlk];   // this run's sum of G conj(H): entry 128 i + j belongs to thread j
+    const int j = threadIdx.x;
+    for (int item = blockIdx.x; item < P * runs; item += gridDim.x) {
+        const int p = item / runs, run = item - p * runs;
+        const int w0 = __ldg(&w_ini[p]), glen = __ldg(&w_len[p]) + L - 1;
+        const int u_end = min(R * n_pair, run_pairs * (run + 1));
+        bool first = true;
+        for (int u = run_pairs * run; u < u_end; u++) {
+            const int r = u / n_pair, b0 = 2 * (u - r * n_pair) * B, b1 = b0 + B;
+            const size_t row = ((size_t)p * R + r) * L;
+            float2 v[16], h[16];
+            if (part) {
+                const float *h0 = rir + row + b0, *h1 = rir + row + b1;
+                const int l0 = min(B, L - b0), l1 = min(B, L - b1);   // (negative: nothing)
+#pragma unroll
+                for (int i = 0; i < 16; i++) {
+                    const int n = j + i * kBlkThreads;
+                    h[i] = make_float2(n < l0 ? __ldg(h0 + n) : 0.0f, n < l1 ? __ldg(h1 + n) : 0.0f);
+                }
+            }
+            {
+                const float *g0 = gt + (size_t)r * n_out + w0 + b0, *g1 = g0 + B;
+                const int l0 = min(B + S - 1, glen - b0), l1 = min(B + S - 1, glen - b1);
+#pragma unroll
+                for (int i = 0; i < 16; i++) {
+                    const int n = j + i * kBlkThreads;
+                    v[i] = make_float2(n < l0 ? __ldg(g0 + n) : 0.0f, n < l1 ? __ldg(g1 + n) : 0.0f);
+                }
+            }
+            if (part) blk_forward(h, buf, W);
+            blk_forward(v, buf, W);
+            if (part) {
+#pragma unroll
+                for (int i = 0; i < 16; i++) {
+                    const float2 a = cmul(v[i], cconj(h[i]));
+                    acc[kBlkThreads * i + j] = first ? a : cadd(acc[kBlkThreads * i + j], a);
+                }
+                first = false;
+            }
+            if (grad_rir) {
+#pragma unroll
+                for (int i = 0; i < 16; i++)
+                    v[i] = cmul(v[i], __ldg(&X[(size_t)p * kBlk + j + kBlkThreads * (i >> 3) + 256 * (i & 7)]));
+                blk_inverse(v, buf, W);
+                float *o0 = grad_rir + row + b0, *o1 = grad_rir + row + b1;
+                const int l0 = min(B, L - b0), l1 = min(B, L - b1);
+#pragma unroll
+                for (int s = 0; s < 16; s++) {
+                    const int n = j + s * kBlkThreads;
+                    const float2 d = v[dr16(s)];
+                    if (n < l0) o0[n] = d.x;
+                    if (n < l1) o1[n] = d.y;
+                }
+            }
+        }
+        if (part) {
+            float2 v[16];
+#pragma unroll
+            for (int i = 0; i < 16; i++) {
+                const float2 a = first ? make_float2(0.0f, 0.0f) : acc[kBlkThreads * i + j];
+                v[i] = make_float2(a.x * (1.0f / kBlk), a.y * (1.0f / kBlk));
+            }
+            blk_inverse(v, buf, W);
+#pragma unroll
+            for (int s = 0; s < 16; s++) {
+                const int n = j + s * kBlkThreads;
+                if (n < S) part[(size_t)item * S + n] = v[dr16(s)].x;
+            }
+        }
+    }
+}
+
+// dL/dx of each point: its runs' parts in order.
+__global__ void blk_sum_kernel(const float *__restrict__ part, const int *__restrict__ w_ini,
+                               const int *__restrict__ w_len, int P, int S, int runs, float *__restrict__ grad_sig) {
+    const int p = blockIdx.y, t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= P || t >= w_len[p]) return;
+    float a = 0.0f;
+    for (int k = 0; k < runs; k++) a += part[((size_t)p * runs + k) * S + t];
+    grad_sig[w_ini[p] + t] = a;
+}
+
+// Layout of the block path's work: lags per block, pairs of blocks per row, runs per point.
+struct BlkPlan {
+    int B, n_pair, runs, run_pairs, grid;
+};
+// For segments up to kBlkMaxSeg (at least half of a block is lags) whose rows do not fit one
+// 2048-point transform anyway.
+bool traj_adjoint_blk_plan(int P, int R, int L, int S, int num_sms, BlkPlan &b) {
+    if (S > kBlkMaxSeg || L + S - 1 <= kBlk || P > 65535) return false;
+    const int most = (kBlk + 1 - S) & ~3;   // blocks start on 16 bytes
+    b.n_pair = (L + 2 * most - 1) / (2 * most);
+    b.B = ((L + 2 * b.n_pair - 1) / (2 * b.n_pair) + 3) & ~3;
+    const long pairs = (long)R * b.n_pair, slots = (long)kBlkPerSm * num_sms;
+    // about four items per resident block, a run of at least two pairs (a run costs one
+    // more inverse transform)
+    b.run_pairs = (int)std::max<long>(std::min<long>(2, pairs), std::min(pairs, P * pairs / (4 * slots)));
+    b.runs = (int)((pairs + b.run_pairs - 1) / b.run_pairs);
+    b.grid = (int)std::min<long>((long)P * b.runs, slots);
+    return true;
+}
+size_t traj_adjoint_blk_floats(const BlkPlan &b, int P, int S) {   // spectra and parts
+    return (size_t)2 * P * kBlk + (size_t)P * b.runs * S;
+}
+int traj_adjoint_blk_fft() { return kBlk; }
+
+cudaError_t traj_adjoint_blk_launch(const double *g, long n_out, const int *w_ini, const int *w_len, const float *seg,
+                                    const float *rir, int P, int R, int L, int S, const BlkPlan &b, const float2 *W,
+                                    float *gt, float *work, float *grad_rir, float *grad_sig, cudaStream_t st) {
+    float2 *X = reinterpret_cast<float2 *>(work);
+    float *part = grad_sig ? work + (size_t)2 * P * kBlk : nullptr;
+    grad_transpose_kernel<<<(unsigned)((n_out + 255) / 256), 256, 0, st>>>(g, n_out, R, gt);
+    if (grad_rir) blk_spectra_kernel<<<std::min(P, b.grid), kBlkThreads, 0, st>>>(seg, P, S, W, X);
+    traj_adjoint_blk_kernel<<<b.grid, kBlkThreads, 0, st>>>(gt, n_out, w_ini, w_len, rir, P, R, L, S, b.B, b.n_pair, b.runs,
+                                                            b.run_pairs, W, X, grad_rir, part);
+    if (grad_sig)
+        blk_sum_kernel<<<dim3((unsigned)((S + 127) / 128), (unsigned)P), 128, 0, st>>>(part, w_ini, w_len, P, S, b.runs,
+                                                                                        grad_sig);
+    return cudaGetLastError();
+}
+
 template <int M>
 static cudaError_t launch_traj_adjoint(const float *gt, long n_out, const int *w_ini, const int *w_len,
                                        const float *rir, int P, int R, int L, const float2 *W,
