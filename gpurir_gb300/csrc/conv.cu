@@ -990,9 +990,46 @@ __device__ __forceinline__ void dft8(float2 &a0, float2 &a1, float2 &a2, float2 
     a3 = cadd(e3, o3); a7 = csub(e3, o3);
 }
 
+// Twiddles of each thread in shared memory, tw[i][j]: the powers 1, 2, 4, 8 of the forward's
+// second pass, 1, 2, 4 of its last pass for both groups, and 1, 2, 4, 8 of the inverse's second
+// and last.  (Read from the size-2048 table in global memory, strides of up to 64 bytes between
+// lanes made them half of the kernel's load wavefronts.)
+constexpr int kBlkTw = 18;
+__device__ __forceinline__ void blk_twiddles(float2 *tw, const float2 *__restrict__ W) {
+    constexpr int T = kBlkThreads;
+    const int j = threadIdx.x;
+    for (int i = 0; i < 4; i++) {
+        tw[i * T + j] = __ldg(&W[((j & 15) * (kBlk / 256)) << i]);
+        tw[(10 + i) * T + j] = __ldg(&W[((j & 7) * (kBlk / 128)) << i]);
+        tw[(14 + i) * T + j] = __ldg(&W[j << i]);
+    }
+    for (int i = 0; i < 3; i++)
+        for (int g = 0; g < 2; g++) tw[(4 + 3 * g + i) * T + j] = __ldg(&W[(j + T * g) << i]);
+    __syncthreads();
+}
+// w^r, r = 1..15, from w, w^2, w^4, w^8 (products of at most three, as twiddle_powers).
+__device__ __forceinline__ void blk_powers(const float2 *tw, float2 (&t)[16]) {
+    constexpr int T = kBlkThreads;
+    const int j = threadIdx.x;
+    t[1] = tw[j];
+    t[2] = tw[T + j];
+    t[4] = tw[2 * T + j];
+    t[8] = tw[3 * T + j];
+    t[3] = cmul(t[1], t[2]);
+    t[5] = cmul(t[1], t[4]);
+    t[6] = cmul(t[2], t[4]);
+    t[7] = cmul(t[3], t[4]);
+    t[9] = cmul(t[1], t[8]);
+    t[10] = cmul(t[2], t[8]);
+    t[11] = cmul(t[3], t[8]);
+    t[12] = cmul(t[4], t[8]);
+    t[13] = cmul(t[5], t[8]);
+    t[14] = cmul(t[6], t[8]);
+    t[15] = cmul(t[7], t[8]);
+}
+
 // Forward transform: v[r] = z[j + 128 r] in, v[8 g + s] = Z[j + 128 g + 256 s] out.
-// W: exp(-2 pi i m / 2048).
-__device__ __forceinline__ void blk_forward(float2 (&v)[16], float2 *buf, const float2 *__restrict__ W) {
+__device__ __forceinline__ void blk_forward(float2 (&v)[16], float2 *buf, const float2 *tw) {
     constexpr int T = kBlkThreads;
     const int j = threadIdx.x;
     dft16<false>(v);
@@ -1005,7 +1042,7 @@ __device__ __forceinline__ void blk_forward(float2 (&v)[16], float2 *buf, const 
     const int k = j & 15;
     {
         float2 t[16];
-        twiddle_powers(W, k * (kBlk / 256), t);
+        blk_powers(tw, t);
 #pragma unroll
         for (int r = 1; r < 16; r++) v[r] = cmul(v[r], t[r]);
     }
@@ -1020,7 +1057,7 @@ __device__ __forceinline__ void blk_forward(float2 (&v)[16], float2 *buf, const 
         float2 *a = v + 8 * g;
 #pragma unroll
         for (int r = 0; r < 8; r++) a[r] = buf[pad16(jj + 256 * r)];
-        const float2 t1 = __ldg(&W[jj]), t2 = __ldg(&W[2 * jj]), t4 = __ldg(&W[4 * jj]);
+        const float2 t1 = tw[(4 + 3 * g) * T + j], t2 = tw[(5 + 3 * g) * T + j], t4 = tw[(6 + 3 * g) * T + j];
         const float2 t3 = cmul(t1, t2);
         a[1] = cmul(a[1], t1);
         a[2] = cmul(a[2], t2);
@@ -1035,7 +1072,7 @@ __device__ __forceinline__ void blk_forward(float2 (&v)[16], float2 *buf, const 
 
 // Inverse transform (unnormalised): v[8 g + s] = Z[j + 128 g + 256 s] in, and out
 // v[dr16(s)] = z[j + 128 s].
-__device__ __forceinline__ void blk_inverse(float2 (&v)[16], float2 *buf, const float2 *__restrict__ W) {
+__device__ __forceinline__ void blk_inverse(float2 (&v)[16], float2 *buf, const float2 *tw) {
     constexpr int T = kBlkThreads;
     const int j = threadIdx.x;
 #pragma unroll
@@ -1054,7 +1091,7 @@ __device__ __forceinline__ void blk_inverse(float2 (&v)[16], float2 *buf, const 
     const int k = j & 7;
     {
         float2 t[16];
-        twiddle_powers(W, k * (kBlk / 128), t);
+        blk_powers(tw + 10 * kBlkThreads, t);
 #pragma unroll
         for (int r = 1; r < 16; r++) v[r] = cmul(v[r], cconj(t[r]));
     }
@@ -1067,7 +1104,7 @@ __device__ __forceinline__ void blk_inverse(float2 (&v)[16], float2 *buf, const 
     for (int r = 0; r < 16; r++) v[r] = buf[pad16(j + r * T)];
     {
         float2 t[16];
-        twiddle_powers(W, j, t);
+        blk_powers(tw + 14 * kBlkThreads, t);
 #pragma unroll
         for (int r = 1; r < 16; r++) v[r] = cmul(v[r], cconj(t[r]));
     }
@@ -1079,7 +1116,9 @@ __device__ __forceinline__ void blk_inverse(float2 (&v)[16], float2 *buf, const 
 __global__ void __launch_bounds__(kBlkThreads) blk_spectra_kernel(const float *__restrict__ seg, int P, int S,
                                                                   const float2 *__restrict__ W, float2 *__restrict__ X) {
     __shared__ __align__(16) float2 buf[kBlk + kBlk / 16];
+    __shared__ float2 tw[kBlkTw * kBlkThreads];
     const int j = threadIdx.x;
+    blk_twiddles(tw, W);
     for (int p = blockIdx.x; p < P; p += gridDim.x) {
         float2 v[16];
 #pragma unroll
@@ -1087,7 +1126,7 @@ __global__ void __launch_bounds__(kBlkThreads) blk_spectra_kernel(const float *_
             const int n = j + r * kBlkThreads;
             v[r] = make_float2(n < S ? __ldg(&seg[(size_t)p * S + n]) : 0.0f, 0.0f);
         }
-        blk_forward(v, buf, W);
+        blk_forward(v, buf, tw);
 #pragma unroll
         for (int i = 0; i < 16; i++)
             X[(size_t)p * kBlk + j + kBlkThreads * (i >> 3) + 256 * (i & 7)] =
@@ -1102,74 +1141,63 @@ __global__ void __launch_bounds__(kBlkThreads, kBlkPerSm) traj_adjoint_blk_kerne
         const float *__restrict__ rir, int P, int R, int L, int S, int B, int n_pair, int runs, int run_pairs,
         const float2 *__restrict__ W, const float2 *__restrict__ X, float *__restrict__ grad_rir,
         float *__restrict__ part) {
-    __shared__ __align__(16) float2 buf[kBlk + kBlk / 16];
-    __shared__ float2 acc[kBlk];   // this run's sum of G conj(H): entry 128 i + j belongs to thread j
+    extern __shared__ __align__(16) float2 sm[];
+    float2 *buf = sm, *tw = buf + kBlk + kBlk / 16;
+    float2 *acc = tw + kBlkTw * kBlkThreads;   // [kBlk] this run's sum of G conj(H): entry 128 i + j is thread j's
     const int j = threadIdx.x;
+    blk_twiddles(tw, W);
     for (int item = blockIdx.x; item < P * runs; item += gridDim.x) {
         const int p = item / runs, run = item - p * runs;
         const int w0 = __ldg(&w_ini[p]), glen = __ldg(&w_len[p]) + L - 1;
-        const int u_end = min(R * n_pair, run_pairs * (run + 1));
-        bool first = true;
-        for (int u = run_pairs * run; u < u_end; u++) {
+        const int u0 = run_pairs * run, u_end = min(R * n_pair, u0 + run_pairs);
+        // the run's pairs, and one more round that inverts its sum of G conj(H) (one body of code
+        // for each transform: unrolled copies of them miss the instruction cache)
+        for (int u = u0; u < u_end + (part ? 1 : 0); u++) {
+            const bool sum = u == u_end;
             const int r = u / n_pair, b0 = 2 * (u - r * n_pair) * B, b1 = b0 + B;
             const size_t row = ((size_t)p * R + r) * L;
+            const int l0 = min(B, L - b0), l1 = min(B, L - b1);   // (negative: nothing)
             float2 v[16], h[16];
-            if (part) {
-                const float *h0 = rir + row + b0, *h1 = rir + row + b1;
-                const int l0 = min(B, L - b0), l1 = min(B, L - b1);   // (negative: nothing)
+            if (sum) {
 #pragma unroll
                 for (int i = 0; i < 16; i++) {
-                    const int n = j + i * kBlkThreads;
-                    h[i] = make_float2(n < l0 ? __ldg(h0 + n) : 0.0f, n < l1 ? __ldg(h1 + n) : 0.0f);
+                    const float2 a = acc[kBlkThreads * i + j];
+                    v[i] = make_float2(a.x * (1.0f / kBlk), a.y * (1.0f / kBlk));
                 }
-            }
-            {
-                const float *g0 = gt + (size_t)r * n_out + w0 + b0, *g1 = g0 + B;
-                const int l0 = min(B + S - 1, glen - b0), l1 = min(B + S - 1, glen - b1);
+            } else {
+#pragma unroll 1
+                for (int side = part ? 0 : 1; side < 2; side++) {   // RIR blocks, then gradient windows
+                    const float *x0 = side ? gt + (size_t)r * n_out + w0 + b0 : rir + row + b0, *x1 = x0 + B;
+                    const int n0 = side ? min(B + S - 1, glen - b0) : l0, n1 = side ? min(B + S - 1, glen - b1) : l1;
 #pragma unroll
-                for (int i = 0; i < 16; i++) {
-                    const int n = j + i * kBlkThreads;
-                    v[i] = make_float2(n < l0 ? __ldg(g0 + n) : 0.0f, n < l1 ? __ldg(g1 + n) : 0.0f);
+                    for (int i = 0; i < 16; i++) {
+                        h[i] = v[i];
+                        const int n = j + i * kBlkThreads;
+                        v[i] = make_float2(n < n0 ? __ldg(x0 + n) : 0.0f, n < n1 ? __ldg(x1 + n) : 0.0f);
+                    }
+                    blk_forward(v, buf, tw);
                 }
-            }
-            if (part) blk_forward(h, buf, W);
-            blk_forward(v, buf, W);
-            if (part) {
+                if (part) {
 #pragma unroll
-                for (int i = 0; i < 16; i++) {
-                    const float2 a = cmul(v[i], cconj(h[i]));
-                    acc[kBlkThreads * i + j] = first ? a : cadd(acc[kBlkThreads * i + j], a);
+                    for (int i = 0; i < 16; i++) {
+                        const float2 a = cmul(v[i], cconj(h[i]));
+                        acc[kBlkThreads * i + j] = u == u0 ? a : cadd(acc[kBlkThreads * i + j], a);
+                    }
                 }
-                first = false;
-            }
-            if (grad_rir) {
+                if (!grad_rir) continue;
 #pragma unroll
                 for (int i = 0; i < 16; i++)
                     v[i] = cmul(v[i], __ldg(&X[(size_t)p * kBlk + j + kBlkThreads * (i >> 3) + 256 * (i & 7)]));
-                blk_inverse(v, buf, W);
-                float *o0 = grad_rir + row + b0, *o1 = grad_rir + row + b1;
-                const int l0 = min(B, L - b0), l1 = min(B, L - b1);
-#pragma unroll
-                for (int s = 0; s < 16; s++) {
-                    const int n = j + s * kBlkThreads;
-                    const float2 d = v[dr16(s)];
-                    if (n < l0) o0[n] = d.x;
-                    if (n < l1) o1[n] = d.y;
-                }
             }
-        }
-        if (part) {
-            float2 v[16];
-#pragma unroll
-            for (int i = 0; i < 16; i++) {
-                const float2 a = first ? make_float2(0.0f, 0.0f) : acc[kBlkThreads * i + j];
-                v[i] = make_float2(a.x * (1.0f / kBlk), a.y * (1.0f / kBlk));
-            }
-            blk_inverse(v, buf, W);
+            blk_inverse(v, buf, tw);
+            float *o0 = sum ? part + (size_t)item * S : grad_rir + row + b0, *o1 = sum ? nullptr : grad_rir + row + b1;
+            const int n0 = sum ? S : l0, n1 = sum ? 0 : l1;
 #pragma unroll
             for (int s = 0; s < 16; s++) {
                 const int n = j + s * kBlkThreads;
-                if (n < S) part[(size_t)item * S + n] = v[dr16(s)].x;
+                const float2 d = v[dr16(s)];
+                if (n < n0) o0[n] = d.x;
+                if (n < n1) o1[n] = d.y;
             }
         }
     }
@@ -1215,8 +1243,15 @@ cudaError_t traj_adjoint_blk_launch(const double *g, long n_out, const int *w_in
     float2 *X = reinterpret_cast<float2 *>(work);
     float *part = grad_sig ? work + (size_t)2 * P * kBlk : nullptr;
     grad_transpose_kernel<<<(unsigned)((n_out + 255) / 256), 256, 0, st>>>(g, n_out, R, gt);
+    const size_t smem = (size_t)(2 * kBlk + kBlk / 16 + kBlkTw * kBlkThreads) * sizeof(float2);
+    static bool attr = false;
+    if (!attr) {
+        cudaError_t e = cudaFuncSetAttribute(traj_adjoint_blk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        attr = true;
+    }
     if (grad_rir) blk_spectra_kernel<<<std::min(P, b.grid), kBlkThreads, 0, st>>>(seg, P, S, W, X);
-    traj_adjoint_blk_kernel<<<b.grid, kBlkThreads, 0, st>>>(gt, n_out, w_ini, w_len, rir, P, R, L, S, b.B, b.n_pair, b.runs,
+    traj_adjoint_blk_kernel<<<b.grid, kBlkThreads, smem, st>>>(gt, n_out, w_ini, w_len, rir, P, R, L, S, b.B, b.n_pair, b.runs,
                                                             b.run_pairs, W, X, grad_rir, part);
     if (grad_sig)
         blk_sum_kernel<<<dim3((unsigned)((S + 127) / 128), (unsigned)P), 128, 0, st>>>(part, w_ini, w_len, P, S, b.runs,
@@ -1298,15 +1333,29 @@ __global__ void ola_kernel(const float *conv, long conv_ld, const int *w_ini, co
     // every p in [lo, e) contributes conv[p][r][t - w_ini[p]]: independent loads, then the
     // compensated sum in increasing p
     float s = 0.0f, comp = 0.0f;
-    const float *col = conv + (long)r * conv_ld + t;
-    const long pstride = (long)R * conv_ld;
-#pragma unroll 4
-    for (int p = lo; p < e; p++) {
-        const float v = __ldg(col + p * pstride - w_ini[p]);
+    auto add = [&](float v) {
         const float y = s + v;                       // two-sum
         const float bb = y - s;
         comp += (s - (y - bb)) + (v - bb);
         s = y;
+    };
+    const float *col = conv + (long)r * conv_ld + t;
+    const long pstride = (long)R * conv_ld;
+    if (uni_w > 0) {   // a constant step from point to point: no index arithmetic per term
+        const long step = pstride - uni_w;
+        const float *q = col + lo * step;
+        int n = e - lo;
+        for (; n >= 8; n -= 8, q += 8 * step) {
+            float v[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) v[k] = __ldg(q + k * step);
+#pragma unroll
+            for (int k = 0; k < 8; k++) add(v[k]);
+        }
+        for (; n > 0; n--, q += step) add(__ldg(q));
+    } else {
+#pragma unroll 4
+        for (int p = lo; p < e; p++) add(__ldg(col + p * pstride - w_ini[p]));
     }
     out[t * R + r] = (double)s + (double)comp;
 }
