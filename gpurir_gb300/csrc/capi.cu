@@ -662,9 +662,8 @@ static int plan_moment(gpurir_sim *s, const std::vector<RoomDesc> &R, Plan &P) {
     const long slots = 2L * s->num_sms;   // (not of a tuned grid: the items fix the results' bits)
     P.mom_T = 1024;
     if (covered / 1024 < slots && images * per_image < 2.0 * covered / 1024 * segment_cost(1024)) P.mom_T = 512;
-    if (moment_cells(P.mom_T, *P.mom) > kMomCells || moment_smem_bytes(P.mom_T, P.axis_cap, *P.mom) > kSmemBudget)
-        P.mom_T = 512;   // (long windows: two blocks per SM)
-    P.mom_smem = moment_smem_bytes(P.mom_T, P.axis_cap, *P.mom);
+    if (moment_cells(P.mom_T, *P.mom) > kMomCells) return fail(GPURIR_ERR_UNSUPPORTED, "window too long");   // (not reached)
+    P.mom_smem = moment_smem_bytes(P.axis_cap, *P.mom);
     int bps = moment_blocks_per_sm(P.mom_smem);
     if (bps < 1) return fail(GPURIR_ERR_CUDA, "ISM kernel does not fit on an SM");
     if (tuning(1) > 0) bps = std::min(bps, tuning(1));   // ism_blocks_per_sm (tuning.cu)
@@ -913,7 +912,6 @@ static int enqueue_kernels(gpurir_sim *s, const Plan &P, const char *d, const La
         m.axis_tab = reinterpret_cast<float4 *>(const_cast<char *>(d) + L.o_axis);
         m.axis_cap = P.axis_cap;
         m.T = P.mom_T;
-        m.nbp = moment_cells(P.mom_T, *P.mom);
         m.win = P.mom_win;
         m.lead = P.mom->lead;
         m.taps = P.mom->taps;
@@ -921,6 +919,8 @@ static int enqueue_kernels(gpurir_sim *s, const Plan &P, const char *d, const La
         m.coef = reinterpret_cast<const float2 *>(d + L.o_coef);
         memcpy(m.run, P.mom->run, sizeof(m.run));
         m.n_quads = P.mom->n_quads;
+        memcpy(m.cut1, P.mom->cut1, sizeof(m.cut1));
+        memcpy(m.cut2, P.mom->cut2, sizeof(m.cut2));
         memcpy(m.S, P.mom->S, sizeof(m.S));
         m.seed = ta.seed; m.offset = ta.offset; m.offset_ptr = ta.offset_ptr;
         m.noise_kind = ta.noise_kind; m.env_out = ta.env_out; m.fuse_tail = ta.fuse; m.tail_pre = ta.pre;

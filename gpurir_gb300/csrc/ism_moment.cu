@@ -56,7 +56,9 @@ namespace gpurir {
 
 constexpr int kMThreads = 384;
 constexpr int kMWarps = kMThreads / 32;
+static_assert(kMWarps == kMomWarps, "");
 constexpr int kMRows = kMThreads;              // image rows per batch
+constexpr int kMStride = kMomCells;            // cells of one array (a constant: offsets are immediates)
 constexpr int kMGroups = 2048;                 // groups of 32 images per batch of rows
 constexpr int kMTwo = 5;                       // pairs of moments with two integers
 constexpr int kMSums = 4 * kMTwo + 2 * (kMPairs - kMTwo) + 1;   // integers per cell, the last one the count
@@ -87,8 +89,8 @@ constexpr int kItemWords = sizeof(IsmItem) / 4, kRoomWords = offsetof(RoomDesc, 
 static_assert(kItemWords <= 32 && kRoomWords <= 64 && kRoomWords > 32, "copied by one warp in one and two loads");
 
 struct MomSmem {
-    int *sum;                 // [kMSums][nbp] moments as integers, and images, per cell;
-                              // then [kMBasis][nbp] float2 and, after those, the filter's parts
+    int *sum;                 // [kMSums][kMStride] moments as integers, and images, per cell;
+                              // then [kMBasis][kMStride] float2 and, after those, the filter's parts
     float2 *coef;             // [8 * quads]: four taps x two output phases
     float4 *rows;             // [kMRows] rho^2 hi, lo, attenuation, m0 | m1 << 16
     int2 *range;              // [kMRows] first image, za | na << 9 | zb << 18
@@ -102,9 +104,9 @@ struct MomSmem {
 __host__ __device__ inline size_t mom_align16(size_t x) { return (x + 15) & ~(size_t)15; }
 
 // Byte offsets of the arrays of MomSmem, in its order; returns the total.
-__host__ __device__ inline size_t mom_layout(int nbp, int n_quads, int axis_cap, size_t o[9]) {
-    const size_t sums = (size_t)kMSums * nbp * sizeof(int);
-    const size_t filt = (size_t)kMBasis * nbp * sizeof(float2) + (size_t)kMWarps * 512 * sizeof(float);
+__host__ __device__ inline size_t mom_layout(int n_quads, int axis_cap, size_t o[9]) {
+    const size_t sums = (size_t)kMSums * kMStride * sizeof(int);
+    const size_t filt = (size_t)kMBasis * kMStride * sizeof(float2) + (size_t)kMWarps * 512 * sizeof(float);
     size_t b = 0;
     o[0] = b; b = mom_align16(b + (sums > filt ? sums : filt));
     o[1] = b; b = mom_align16(b + (size_t)n_quads * 8 * sizeof(float2));
@@ -362,7 +364,7 @@ __global__ void __launch_bounds__(kMThreads, 2) ism_moment_kernel(const __grid_c
     MomSmem s;
     {
         size_t o[9];
-        mom_layout(P.nbp, P.n_quads, P.axis_cap, o);
+        mom_layout(P.n_quads, P.axis_cap, o);
         s.sum = reinterpret_cast<int *>(smem_raw + o[0]);
         s.coef = reinterpret_cast<float2 *>(smem_raw + o[1]);
         s.rows = reinterpret_cast<float4 *>(smem_raw + o[2]);
@@ -374,8 +376,8 @@ __global__ void __launch_bounds__(kMThreads, 2) ism_moment_kernel(const __grid_c
         s.tab = P.axis_cap <= kMTabSmem ? reinterpret_cast<float4 *>(smem_raw + o[8])
                                         : P.axis_tab + (size_t)(2 * blockIdx.x) * P.axis_cap;
     }
-    float2 *basis = reinterpret_cast<float2 *>(s.sum);                 // [kMBasis][nbp]
-    float *part = reinterpret_cast<float *>(basis + kMBasis * P.nbp);  // filter parts
+    float2 *basis = reinterpret_cast<float2 *>(s.sum);                 // [kMBasis][kMStride]
+    float *part = reinterpret_cast<float *>(basis + kMBasis * kMStride);  // filter parts
     int *ctl = s.red + 32;   // [0] most images of a cell, [1] last cell with an image, [2] loud images
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const unsigned le_mask = 0xffffffffu >> (31 - lane);
@@ -417,7 +419,7 @@ __global__ void __launch_bounds__(kMThreads, 2) ism_moment_kernel(const __grid_c
         const int len = t_hi - t_lo;
         const int tiles = (len + 511) >> 9;
         const int nb = ((len + 1) >> 1) + P.taps - 1;         // cells whose taps reach the segment
-        const int nbe = min(P.nbp, tiles * 256 + 4 * P.quads + 8);      // cells the filter reads
+        const int nbe = min(kMStride, tiles * 256 + 4 * P.quads + 8);      // cells the filter reads
         const bool last = t_hi == C.it.t_hi;
         __syncthreads();   // tables written; the previous segment's output is done with the shared arrays
         if (last && warp == 0) ctx_item(s.ctx[par ^ 1], P, next, lane);
@@ -470,8 +472,9 @@ __global__ void __launch_bounds__(kMThreads, 2) ism_moment_kernel(const __grid_c
                 const float scale = __int_as_float((127 + k) << 23), most = __int_as_float((127 + 20 - shift) << 23);
                 const float fine = most;       // steps of the second integer in one of the first
                 unit = __int_as_float((127 - k) << 23);
-                for (int i = tid; i < kMSums * P.nbp / 4; i += kMThreads)
-                    reinterpret_cast<int4 *>(s.sum)[i] = make_int4(0, 0, 0, 0);
+                for (int a = warp; a < kMSums; a += kMWarps)
+                    for (int i = lane; 4 * i < nbe; i += 32)
+                        reinterpret_cast<int4 *>(s.sum + a * kMStride)[i] = make_int4(0, 0, 0, 0);
                 if (tid < 3) ctl[tid] = tid == 1 ? -1 : 0;
                 __syncthreads();
                 for (int rbase = 0; rbase < my_rows; rbase += batch) {
@@ -551,18 +554,18 @@ __global__ void __launch_bounds__(kMThreads, 2) ism_moment_kernel(const __grid_c
                             continue;
                         }
                         int *cell = s.sum + b;
-                        atomicAdd(cell + (kMSums - 1) * P.nbp, 1);
+                        atomicAdd(cell + (kMSums - 1) * kMStride, 1);
                         const float2 m2f = make_float2(kMMagic, kMMagic), n2f = make_float2(-kMMagic, -kMMagic);
                         image_moments(q, u, [&](int p, float2 v) {
                             const float2 t = add2_rn(v, m2f);
-                            int *c = cell + (p < kMTwo ? 4 * p : 4 * kMTwo + 2 * (p - kMTwo)) * P.nbp;
+                            int *c = cell + (p < kMTwo ? 4 * p : 4 * kMTwo + 2 * (p - kMTwo)) * kMStride;
                             atomicAdd(c, __float_as_int(t.x));
-                            atomicAdd(c + P.nbp, __float_as_int(t.y));
+                            atomicAdd(c + kMStride, __float_as_int(t.y));
                             if (p < kMTwo) {   // what the rounding left, in steps of 1 / fine
                                 const float2 rest = __ffma2_rn(add2_rn(t, n2f), make_float2(-1.0f, -1.0f), v);
                                 const float2 w = __ffma2_rn(rest, make_float2(fine, fine), m2f);
-                                atomicAdd(c + 2 * P.nbp, __float_as_int(w.x));
-                                atomicAdd(c + 3 * P.nbp, __float_as_int(w.y));
+                                atomicAdd(c + 2 * kMStride, __float_as_int(w.x));
+                                atomicAdd(c + 3 * kMStride, __float_as_int(w.y));
                             }
                         });
                     }
@@ -570,7 +573,7 @@ __global__ void __launch_bounds__(kMThreads, 2) ism_moment_kernel(const __grid_c
                 __syncthreads();   // sums complete
                 int n_max = 0, top = -1;
                 for (int b = tid; b < nbe; b += kMThreads) {
-                    const int n = s.sum[(kMSums - 1) * P.nbp + b];
+                    const int n = s.sum[(kMSums - 1) * kMStride + b];
                     n_max = max(n_max, n);
                     if (n > 0) top = b;
                 }
@@ -597,17 +600,17 @@ __global__ void __launch_bounds__(kMThreads, 2) ism_moment_kernel(const __grid_c
                 const int b = tid + i * kMThreads;
 #pragma unroll
                 for (int p = 0; p < kMBasis; p++) F[i][p] = make_float2(0.0f, 0.0f);
-                const int n = b < nbe ? s.sum[(kMSums - 1) * P.nbp + b] : 0;
+                const int n = b < nbe ? s.sum[(kMSums - 1) * kMStride + b] : 0;
                 if (b >= nbe || (n == 0 && n_loud == 0)) continue;
                 const int bias = n * kMMagicBits;   // (modulo 2^32, as the sums)
                 float2 A[kMPairs];
 #pragma unroll
                 for (int p = 0; p < kMPairs; p++) {
-                    const int *c = s.sum + (p < kMTwo ? 4 * p : 4 * kMTwo + 2 * (p - kMTwo)) * P.nbp + b;
-                    A[p] = make_float2((float)(c[0] - bias), (float)(c[P.nbp] - bias));
+                    const int *c = s.sum + (p < kMTwo ? 4 * p : 4 * kMTwo + 2 * (p - kMTwo)) * kMStride + b;
+                    A[p] = make_float2((float)(c[0] - bias), (float)(c[kMStride] - bias));
                     if (p < kMTwo) {
-                        A[p].x = fmaf((float)(c[2 * P.nbp] - bias), fine, A[p].x);
-                        A[p].y = fmaf((float)(c[3 * P.nbp] - bias), fine, A[p].y);
+                        A[p].x = fmaf((float)(c[2 * kMStride] - bias), fine, A[p].x);
+                        A[p].y = fmaf((float)(c[3 * kMStride] - bias), fine, A[p].y);
                     }
                     A[p].x *= unit;
                     A[p].y *= unit;
@@ -631,7 +634,7 @@ __global__ void __launch_bounds__(kMThreads, 2) ism_moment_kernel(const __grid_c
                 const int b = tid + i * kMThreads;
                 if (b < nbe)
 #pragma unroll
-                    for (int p = 0; p < kMBasis; p++) basis[p * P.nbp + 2 * mchunk(b >> 1) + (b & 1)] = F[i][p];
+                    for (int p = 0; p < kMBasis; p++) basis[p * kMStride + 2 * mchunk(b >> 1) + (b & 1)] = F[i][p];
             }
             __syncthreads();
         }
@@ -646,13 +649,14 @@ __global__ void __launch_bounds__(kMThreads, 2) ism_moment_kernel(const __grid_c
                 float2 acc[16];
 #pragma unroll
                 for (int e = 0; e < 16; e++) acc[e] = make_float2(0.0f, 0.0f);
-                int q = P.n_quads * g / G;
-                const int q_end = P.n_quads * (g + 1) / G;
+                const unsigned char *cut = act == 1 ? P.cut1 : P.cut2;
+                int q = cut[g];
+                const int q_end = cut[g + 1];
                 int r = 0, base = 0;
                 while (q < q_end) {
                     while (q >= base + P.run[r].quads) base += P.run[r++].quads;
                     const int run = min(q_end, base + P.run[r].quads) - q;
-                    const float2 *pair = basis + P.run[r].pair * P.nbp;
+                    const float2 *pair = basis + P.run[r].pair * kMStride;
                     const float2 *cf = s.coef + 8 * q;
                     int quad = 2 * (32 * tile + lane) + P.run[r].first + (q - base);
                     float2 qa[4], qb[4], qc[4];
@@ -1016,6 +1020,32 @@ void moment_basis(int tw, MomBasis &B) {
         }
 }
 
+// Cuts of the filter's quads into G ranges of about equal time: a quad, and a good one more
+// for every run that a range touches (its first cells are loaded before it starts).
+static void cut_filter(const MomBasis &B, int G, unsigned char *cut) {
+    std::vector<int> begin(B.n_quads, 0);   // 1: a run begins at this quad
+    for (int r = 0, q = 0; r < B.n_runs; q += B.run[r++].quads) begin[q] = 1;
+    for (double most = (double)B.n_quads / G;; most += 0.1) {
+        int g = 0;
+        double c = 0.0;
+        cut[0] = 0;
+        for (int q = 0; q < B.n_quads; q++) {
+            const double add = 1.0 + (begin[q] || q == cut[g] ? 1.3 : 0.0);
+            if (q > cut[g] && c + add > most) {
+                if (++g == G) break;
+                cut[g] = (unsigned char)q;
+                c = 2.3;
+            } else {
+                c += add;
+            }
+        }
+        if (g < G) {
+            while (g < G) cut[++g] = (unsigned char)B.n_quads;
+            return;
+        }
+    }
+}
+
 // Bases of the window lengths in use, built once each (about 1 ms).
 const MomBasis &moment_basis_cached(int tw) {
     static std::mutex mu;
@@ -1025,6 +1055,8 @@ const MomBasis &moment_basis_cached(int tw) {
     if (it == known.end()) {
         it = known.emplace(tw, MomBasis{}).first;
         moment_basis(tw, it->second);
+        cut_filter(it->second, kMWarps, it->second.cut1);
+        cut_filter(it->second, kMWarps / 2, it->second.cut2);
     }
     return it->second;
 }
@@ -1032,9 +1064,9 @@ const MomBasis &moment_basis_cached(int tw) {
 // cells of a launch: the longest segment's outputs and the filter's reach past them
 int moment_cells(int T, const MomBasis &B) { return (T / 2 + 4 * B.quads + 8 + 7) / 8 * 8; }
 
-size_t moment_smem_bytes(int T, int axis_cap, const MomBasis &B) {
+size_t moment_smem_bytes(int axis_cap, const MomBasis &B) {
     size_t o[9];
-    return mom_layout(moment_cells(T, B), B.n_quads, axis_cap, o);
+    return mom_layout(B.n_quads, axis_cap, o);
 }
 
 int moment_blocks_per_sm(size_t smem) {

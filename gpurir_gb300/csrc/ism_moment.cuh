@@ -14,6 +14,7 @@ constexpr double kMomNear = 4.6;          // taps beyond this one pairs 0 to 2
 constexpr int kMomMinTw = 48;             // window lengths the moment path is used for
 constexpr int kMomMaxTw = 400;
 constexpr int kMomCells = 768;            // most cells of a segment
+constexpr int kMomWarps = 12;             // warps of a block
 constexpr int kMomRuns = 18;               // three per pair
 
 // Quads (groups of four cell taps) of one basis pair.
@@ -28,6 +29,7 @@ struct MomBasis {
     float2 S[kMBasis][kMPairs];           // moments -> basis
     MomRun run[kMomRuns];
     int n_runs = 0, n_quads = 0;          // over all runs
+    unsigned char cut1[kMomWarps + 1], cut2[kMomWarps / 2 + 1];   // the warps' ranges of quads, for one tile or two
     std::vector<float2> coef;             // 8 n_quads: per quad, tap by tap, two output phases
 };
 
@@ -40,12 +42,13 @@ struct MomLaunch {
     int *work_counter, *status;
     float4 *axis_tab;                 // per block: two tables of axis_cap entries
     int axis_cap;
-    int T, nbp;                       // longest segment, cells
+    int T;                            // longest segment
     int win;                          // shortest last segment of an item (holds the envelope window)
     int lead, taps, quads;            // as in MomBasis
     const float2 *coef;
     MomRun run[kMomRuns];
     int n_quads;
+    unsigned char cut1[kMomWarps + 1], cut2[kMomWarps / 2 + 1];
     float2 S[kMBasis][kMPairs];
     // diffuse tail of the RIRs whose last segment is one item (TailArgs)
     uint64_t seed, offset;
@@ -58,7 +61,7 @@ struct MomLaunch {
 
 const MomBasis &moment_basis_cached(int tw);
 int moment_cells(int T, const MomBasis &B);
-size_t moment_smem_bytes(int T, int axis_cap, const MomBasis &B);
+size_t moment_smem_bytes(int axis_cap, const MomBasis &B);
 int moment_blocks_per_sm(size_t smem);
 cudaError_t moment_launch(const MomLaunch &p, size_t smem, int grid, cudaStream_t st);
 
