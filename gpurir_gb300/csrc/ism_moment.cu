@@ -62,6 +62,12 @@ constexpr int kMStride = kMomCells;            // cells of one array (a constant
 constexpr int kMGroups = 2048;                 // groups of 32 images per batch of rows
 constexpr int kMTwo = 5;                       // pairs of moments with two integers
 constexpr int kMSums = 4 * kMTwo + 2 * (kMPairs - kMTwo) + 1;   // integers per cell, the last one the count
+// Packed sums, for cells of fewer than 7/8 2^h images (h <= 9).  Amplitudes span 2^21 steps.
+// T0..T7: two words of steps and, shared by a pair, one with what the rounding left, 16 bits
+// each; T8..T10: a word each; T11 above a count of 10 bits; T12 (17 bits) above T13 (15 bits).
+constexpr int kMPTwo = 4, kMPSums = 3 * kMPTwo + 2 + 3;
+constexpr int kMPSpan = 21, kMPCount = 10, kMPMinBits = 6, kMPMaxBits = 9;
+static_assert(kMPairs == 7, "the packed words are laid out for fourteen moments");
 constexpr int kMLoud = 32;                     // images of a segment above the bound of its scale
 constexpr int kMTabSmem = 256;                 // per-axis entries of a launch held in shared memory
 constexpr float kMMagic = 12582912.0f;         // 1.5 2^23
@@ -81,8 +87,7 @@ struct MomCtx {
     float pos[6], ori[6];                               // source, receiver; their unit axes (zero: omni)
     float inv_L[3], ov[3], p2, q2, inv_k;               // reciprocals, source overhang, offsets along the last axis
     int reach;                                          // last sample an image of the pair can have
-    int att[3], near2[3];                               // bits of the largest |attenuation| and of the least
-                                                        // squared component along each axis
+    int near2[3];                                       // bits of the least squared component along each axis
     int valid;
 };
 constexpr int kItemWords = sizeof(IsmItem) / 4, kRoomWords = offsetof(RoomDesc, pw) / 4;
@@ -97,7 +102,7 @@ struct MomSmem {
     unsigned short *group;    // [kMGroups] row of a group's first image
     float4 *loud;             // [kMLoud] a, u, cell
     MomCtx *ctx;              // [2]
-    int *red;                 // scan scratch [32], control words [8]
+    int *red;                 // scan scratch [32], control words [16]
     float4 *tab;              // [2][axis_cap] per-axis tables (or in global memory)
 };
 
@@ -115,7 +120,7 @@ __host__ __device__ inline size_t mom_layout(int n_quads, int axis_cap, size_t o
     o[4] = b; b = b + kMGroups * sizeof(unsigned short);
     o[5] = b; b = b + kMLoud * sizeof(float4);
     o[6] = b; b = mom_align16(b + 2 * sizeof(MomCtx));
-    o[7] = b; b = mom_align16(b + 40 * sizeof(int));
+    o[7] = b; b = mom_align16(b + 48 * sizeof(int));
     o[8] = b; b += axis_cap <= kMTabSmem ? 2 * (size_t)axis_cap * sizeof(float4) : 0;
     return b;
 }
@@ -267,7 +272,6 @@ __device__ __forceinline__ void ctx_finish(MomCtx &c, const MomLaunch &P, int id
         const float L = R.L[lane], sa = c.pos[lane], ra = c.pos[3 + lane], inv = 1.0f / L;
         float v2min;
         axis_extent(R.nb[lane], L, sa, ra, v2min, v2);
-        c.att[lane] = 0;
         c.near2[lane] = 0x7f7fffff;
         c.inv_L[lane] = inv;
         c.ov[lane] = fmaxf(fmaxf(-sa, sa - L), 0.0f);
@@ -298,7 +302,6 @@ __device__ __forceinline__ void axis_tables(const MomLaunch &P, MomCtx &c, float
         int ca, fa;
         image_axis(m, R.nb[a], ca, fa);
         const float att = G.pw[2 * a][abs(ca - fa)] * G.pw[2 * a + 1][abs(ca)];
-        atomicMax(&c.att[a], __float_as_int(fabsf(att)));
         const float La = R.L[a], sa = c.pos[a], ra = c.pos[3 + a];
         if (R.ref_delay) {   // the reference's float32 component; its square only bounds
             const float v = ref_axis_component(ca, fa, La, sa, ra);
@@ -378,7 +381,8 @@ __global__ void __launch_bounds__(kMThreads, 2) ism_moment_kernel(const __grid_c
     }
     float2 *basis = reinterpret_cast<float2 *>(s.sum);                 // [kMBasis][kMStride]
     float *part = reinterpret_cast<float *>(basis + kMBasis * kMStride);  // filter parts
-    int *ctl = s.red + 32;   // [0] most images of a cell, [1] last cell with an image, [2] loud images
+    int *ctl = s.red + 32;   // [0] most images of a cell, [1] last cell with an image, [2] loud images,
+                             // [3..8] bounds of |attenuation| along the axes, [9] images not counted in a cell
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const unsigned le_mask = 0xffffffffu >> (31 - lane);
     for (int i = tid; i < 8 * P.n_quads; i += kMThreads) s.coef[i] = P.coef[i];
@@ -443,40 +447,63 @@ __global__ void __launch_bounds__(kMThreads, 2) ism_moment_kernel(const __grid_c
             }
             const float rW1 = 1.0f / (float)max(W1, 1);
             const int batch = min(kMRows, 32 * kMGroups / N2);   // rows at once: their images fill the groups at most
-            float att_max = __int_as_float(C.att[0]) * __int_as_float(C.att[1]) * __int_as_float(C.att[2]);
-            if (!(att_max <= 1.0f)) {   // walls that amplify: the bound of this segment's indices alone
-                int a2, b2;
-                axis_range(N2, inv_L2, C.ov[2], C.pos[5], d_hi, a2, b2);
-                const int lo[3] = {a0, N0 + a1, N0 + N1 + a2};
-                const int hi[3] = {a0 + (W1 > 0 ? n_box / W1 : 0), N0 + a1 + W1, N0 + N1 + b2};
-                if (tid < 3) ctl[3 + tid] = 0;
-                __syncthreads();
-#pragma unroll
-                for (int a = 0; a < 3; a++)
-                    for (int e = lo[a] + tid; e < hi[a]; e += kMThreads)
-                        atomicMax(&ctl[3 + a], __float_as_int(fabsf(tab[e].w)));
-                __syncthreads();
-                att_max = __int_as_float(ctl[3]) * __int_as_float(ctl[4]) * __int_as_float(ctl[5]);
-            }
+            // mean images per cell at the segment's end: a room's volume holds one; cells with few
+            // have packed sums
+            const float mean = 25.14f * d_hi * d_hi * C.inv_k * C.inv_L[0] * C.inv_L[1] * inv_L2 / (float)C.it.i_hi;
+            int bits = kMPMinBits;
+            while (bits < kMPMaxBits && 4.0f * mean + 24.0f > (float)(7 << bits >> 3)) bits++;
+            bool packed = 2.0f * mean + 24.0f <= (float)(7 << bits >> 3);
             float unit;        // value of one step of a sum's first integer
             int shift = 0;     // bits given up to hold more images per cell
-            for (int round = 0;; round++) {
-                // scale: amplitudes are at most att_max / (4 pi d) with d the shell's inner radius or
-                // the nearest image's distance; at first images nearer than 5 cm are left to the
-                // loud list.  2^(e + 1) bounds them; 2^(20 - shift) steps span that.
+            for (int round = 0;;) {
+                const int words = packed ? kMPSums : kMSums;
+                for (int a = warp; a < words; a += kMWarps)
+                    for (int i = lane; 4 * i < nbe; i += 32)
+                        reinterpret_cast<int4 *>(s.sum + a * kMStride)[i] = make_int4(0, 0, 0, 0);
+                if (warp < 3) {   // largest |attenuation| along one axis, and beyond d_lo / sqrt(3)
+                    int a2, b2;
+                    axis_range(N2, inv_L2, C.ov[2], C.pos[5], d_hi, a2, b2);
+                    const int lo = warp == 0 ? a0 : (warp == 1 ? N0 + a1 : N0 + N1 + a2);
+                    const int hi = warp == 0 ? a0 + (W1 > 0 ? n_box / W1 : 0) : (warp == 1 ? N0 + a1 + W1 : N0 + N1 + b2);
+                    const float far2 = 0.3333f * dlo2;
+                    int full = 0, far = 0;
+                    for (int i = lo + lane; i < hi; i += 32) {
+                        const int w = __float_as_int(fabsf(tab[i].w));
+                        full = max(full, w);
+                        if (!(tab[i].x < far2)) far = max(far, w);
+                    }
+                    full = __reduce_max_sync(0xffffffffu, full);
+                    far = __reduce_max_sync(0xffffffffu, far);
+                    if (lane == 0) {
+                        ctl[3 + warp] = full;
+                        ctl[6 + warp] = far;
+                    }
+                } else if (warp == 3) {
+                    if (lane < 3) ctl[lane] = lane == 1 ? -1 : 0;
+                    if (lane == 3) ctl[9] = 0;
+                }
+                __syncthreads();
+                // scale: of an image at least d_lo away one component is d_lo / sqrt(3) at least, which bounds
+                // its attenuation (walls that amplify too), and amplitudes are at most that bound over
+                // 4 pi d with d the shell's inner radius or the nearest image's distance; at first images
+                // nearer than 5 cm are left to the loud list.  2^(e + 1) bounds them; the span of the steps
+                // (2^(20 - shift), 2^21 packed) covers that.
+                float att_max;
+                {
+                    const float f0 = __int_as_float(ctl[3]), f1 = __int_as_float(ctl[4]), f2 = __int_as_float(ctl[5]);
+                    att_max = fmaxf(fmaxf(__int_as_float(ctl[6]) * (f1 * f2), __int_as_float(ctl[7]) * (f0 * f2)),
+                                    __int_as_float(ctl[8]) * (f0 * f1));
+                }
                 const float first = sqrtf(__int_as_float(C.near2[0]) + __int_as_float(C.near2[1]) +
                                           __int_as_float(C.near2[2])) * 0.999f;
                 const float near = fmaxf(fmaxf(d_lo, first), round == 0 ? 0.05f : 1.0e-12f);
                 const int e = (__float_as_int(att_max * 0.0797f / near) >> 23) - 127;
-                const int k = min(max(19 - shift - e, -120), 120);
-                const float scale = __int_as_float((127 + k) << 23), most = __int_as_float((127 + 20 - shift) << 23);
-                const float fine = most;       // steps of the second integer in one of the first
+                const int span = packed ? kMPSpan : 20 - shift;
+                const int k = min(max(span - 1 - e, -120), 120);
+                const float scale = __int_as_float((127 + k) << 23), most = __int_as_float((127 + span) << 23);
+                const float fine = packed ? __int_as_float((127 + 16 - bits) << 23) : most;   // steps of the second integer in one of the first
                 unit = __int_as_float((127 - k) << 23);
-                for (int a = warp; a < kMSums; a += kMWarps)
-                    for (int i = lane; 4 * i < nbe; i += 32)
-                        reinterpret_cast<int4 *>(s.sum + a * kMStride)[i] = make_int4(0, 0, 0, 0);
-                if (tid < 3) ctl[tid] = tid == 1 ? -1 : 0;
-                __syncthreads();
+                int placed = 0;
                 for (int rbase = 0; rbase < my_rows; rbase += batch) {
                     // ---- one row per thread: its m2 ranges [za, ya) and [zb, yb)
                     int za = 0, ya = 0, zb = 0, yb = 0;
@@ -554,16 +581,35 @@ __global__ void __launch_bounds__(kMThreads, 2) ism_moment_kernel(const __grid_c
                             continue;
                         }
                         int *cell = s.sum + b;
-                        atomicAdd(cell + (kMSums - 1) * kMStride, 1);
                         const float2 m2f = make_float2(kMMagic, kMMagic), n2f = make_float2(-kMMagic, -kMMagic);
+                        const float2 fine2 = make_float2(fine, fine), minus = make_float2(-1.0f, -1.0f);
+                        if (packed) {
+                            placed++;
+                            const float f11 = __int_as_float((127 - bits) << 23);
+                            image_moments(q, u, [&](int p, float2 v) {
+                                int *c = cell + (p < kMPTwo ? 3 * p : 3 * kMPTwo + 2 * (p - kMPTwo)) * kMStride;
+                                const float2 f = p == 5 ? make_float2(1.0f, f11)
+                                                        : make_float2(f11 * 0.03125f, f11 * 0.0078125f);
+                                const float2 t = p < 5 ? add2_rn(v, m2f) : __ffma2_rn(v, f, m2f);
+                                const unsigned x = __float_as_uint(t.x), y = __float_as_uint(t.y);
+                                // (the constant's bits are zero below bit 22: shifted by ten or more they vanish)
+                                atomicAdd(c, (int)(p == 6 ? (x << 15) + y : x));
+                                if (p < 6) atomicAdd(c + kMStride, (int)(p == 5 ? (y << kMPCount) + 1 : y));
+                                if (p < kMPTwo) {   // what the rounding left, in steps of 1 / fine
+                                    const float2 w = __ffma2_rn(__ffma2_rn(add2_rn(t, n2f), minus, v), fine2, m2f);
+                                    atomicAdd(c + 2 * kMStride, (int)((__float_as_uint(w.x) << 16) + __float_as_uint(w.y)));
+                                }
+                            });
+                            continue;
+                        }
+                        atomicAdd(cell + (kMSums - 1) * kMStride, 1);
                         image_moments(q, u, [&](int p, float2 v) {
                             const float2 t = add2_rn(v, m2f);
                             int *c = cell + (p < kMTwo ? 4 * p : 4 * kMTwo + 2 * (p - kMTwo)) * kMStride;
                             atomicAdd(c, __float_as_int(t.x));
                             atomicAdd(c + kMStride, __float_as_int(t.y));
-                            if (p < kMTwo) {   // what the rounding left, in steps of 1 / fine
-                                const float2 rest = __ffma2_rn(add2_rn(t, n2f), make_float2(-1.0f, -1.0f), v);
-                                const float2 w = __ffma2_rn(rest, make_float2(fine, fine), m2f);
+                            if (p < kMTwo) {
+                                const float2 w = __ffma2_rn(__ffma2_rn(add2_rn(t, n2f), minus, v), fine2, m2f);
                                 atomicAdd(c + 2 * kMStride, __float_as_int(w.x));
                                 atomicAdd(c + 3 * kMStride, __float_as_int(w.y));
                             }
@@ -572,48 +618,77 @@ __global__ void __launch_bounds__(kMThreads, 2) ism_moment_kernel(const __grid_c
                 }
                 __syncthreads();   // sums complete
                 int n_max = 0, top = -1;
+                const int *count = s.sum + (packed ? 3 * kMPTwo + 3 : kMSums - 1) * kMStride;
                 for (int b = tid; b < nbe; b += kMThreads) {
-                    const int n = s.sum[(kMSums - 1) * kMStride + b];
+                    const int n = packed ? count[b] & ((1 << kMPCount) - 1) : count[b];
                     n_max = max(n_max, n);
+                    placed -= n;
                     if (n > 0) top = b;
                 }
                 for (int l = 0; l < min(ctl[2], kMLoud); l++) top = max(top, __float_as_int(s.loud[l].z));
                 n_max = __reduce_max_sync(0xffffffffu, n_max);
                 top = __reduce_max_sync(0xffffffffu, top);
+                placed = __reduce_add_sync(0xffffffffu, placed);
                 if (lane == 0) {
                     atomicMax(&ctl[0], n_max);
                     atomicMax(&ctl[1], top);
+                    atomicAdd(&ctl[9], placed);
                 }
                 __syncthreads();
-                // a cell's sums hold 2^(11 + shift) images
-                if (round > 0 || (ctl[0] < 2048 && ctl[2] <= kMLoud)) break;
-                while (ctl[0] >> (11 + shift)) shift++;
+                if (packed) {   // too many images in a cell, or more than its count holds: unpacked sums
+                    if (ctl[0] <= (7 << bits >> 3) && ctl[9] == 0 && ctl[2] <= kMLoud) break;
+                    packed = false;
+                } else {        // a cell's sums hold 2^(11 + shift) images
+                    if (round > 0 || (ctl[0] < 2048 && ctl[2] <= kMLoud)) break;
+                    while (ctl[0] >> (11 + shift)) shift++;
+                    round++;
+                }
                 __syncthreads();
             }
             const int n_loud = ctl[2];
             act = ctl[1] >= 0 ? min((ctl[1] >> 8) + 1, tiles) : 0;
             // ---- sums -> basis, each cell by one thread
-            const float fine = __int_as_float((127 - 20 + shift) << 23);
+            const float fine = __int_as_float((127 - (packed ? 16 - bits : 20 - shift)) << 23);
             float2 F[2][kMBasis];
 #pragma unroll
             for (int i = 0; i < 2; i++) {
                 const int b = tid + i * kMThreads;
 #pragma unroll
                 for (int p = 0; p < kMBasis; p++) F[i][p] = make_float2(0.0f, 0.0f);
-                const int n = b < nbe ? s.sum[(kMSums - 1) * kMStride + b] : 0;
+                const int *sum = s.sum + b;
+                const int tc = b < nbe ? sum[(packed ? 3 * kMPTwo + 3 : kMSums - 1) * kMStride] : 0;
+                const int n = packed ? tc & ((1 << kMPCount) - 1) : tc;
                 if (b >= nbe || (n == 0 && n_loud == 0)) continue;
                 const int bias = n * kMMagicBits;   // (modulo 2^32, as the sums)
                 float2 A[kMPairs];
+                if (packed) {
 #pragma unroll
-                for (int p = 0; p < kMPairs; p++) {
-                    const int *c = s.sum + (p < kMTwo ? 4 * p : 4 * kMTwo + 2 * (p - kMTwo)) * kMStride + b;
-                    A[p] = make_float2((float)(c[0] - bias), (float)(c[kMStride] - bias));
-                    if (p < kMTwo) {
-                        A[p].x = fmaf((float)(c[2 * kMStride] - bias), fine, A[p].x);
-                        A[p].y = fmaf((float)(c[3 * kMStride] - bias), fine, A[p].y);
+                    for (int p = 0; p < kMPTwo; p++) {
+                        const int *c = sum + 3 * p * kMStride;
+                        const int w = c[2 * kMStride] - bias, y = (short)w;
+                        A[p] = make_float2(fmaf((float)((w - y) >> 16), fine, (float)(c[0] - bias)),
+                                           fmaf((float)y, fine, (float)(c[kMStride] - bias)));
                     }
-                    A[p].x *= unit;
-                    A[p].y *= unit;
+                    const int *c = sum + 3 * kMPTwo * kMStride;
+                    const float f11 = __int_as_float((127 + bits) << 23);
+                    A[4] = make_float2((float)(c[0] - bias), (float)(c[kMStride] - bias));
+                    A[5] = make_float2((float)(c[2 * kMStride] - bias), (float)(tc >> kMPCount) * f11);
+                    const int w = c[4 * kMStride] - bias, y = (int)((unsigned)w << 17) >> 17;
+                    A[6] = make_float2((float)((w - y) >> 15) * (f11 * 32.0f), (float)y * (f11 * 128.0f));
+#pragma unroll
+                    for (int p = 0; p < kMPairs; p++) A[p] = __fmul2_rn(A[p], make_float2(unit, unit));
+                } else {
+#pragma unroll
+                    for (int p = 0; p < kMPairs; p++) {
+                        const int *c = sum + (p < kMTwo ? 4 * p : 4 * kMTwo + 2 * (p - kMTwo)) * kMStride;
+                        A[p] = make_float2((float)(c[0] - bias), (float)(c[kMStride] - bias));
+                        if (p < kMTwo) {
+                            A[p].x = fmaf((float)(c[2 * kMStride] - bias), fine, A[p].x);
+                            A[p].y = fmaf((float)(c[3 * kMStride] - bias), fine, A[p].y);
+                        }
+                        A[p].x *= unit;
+                        A[p].y *= unit;
+                    }
                 }
                 if (n_loud > kMLoud) {   // amplitudes past any finite bound: as such sums end in FP32
                     A[0].x = A[0].y = __int_as_float(0x7fffffff);

@@ -75,6 +75,19 @@ def test_more_images_per_cell_than_the_sums_hold(built):
     _check(room, np.full(6, 0.97, np.float32), ps, pr, [101, 101, 101], 0.073, 16000.0, pairs=[(0, 0), (19, 15)])
 
 
+@pytest.mark.parametrize("centred", [False, True])   # True: many images of one delay, cells past the packed sums
+@pytest.mark.parametrize("edge", [3.0, 2.0, 1.5, 1.2, 1.0])
+def test_packed_sums(built, edge, centred):
+    """Cells of 15 to 400 images: each width of the packed sums, both sides of the last one."""
+    room = [edge, edge, edge] if centred else [edge, 1.1 * edge, 0.9 * edge]
+    ps, pr, beta = _scene(int(10 * edge), room, 20, 16)
+    if centred:
+        ps[0] = pr[0] = 0.5 * edge
+        pr[0, 0] += np.float32(0.06)
+    n = int(2 * 27.0 / edge) + 3
+    _check(room, beta, ps, pr, [n, n, n + 4], 0.08, 16000.0, pairs=[(0, 0), (19, 15)])
+
+
 @pytest.mark.parametrize("gap", [1e-4, 0.01, 0.049])
 def test_source_next_to_the_receiver(built, gap):
     """Direct paths below the 5 cm of the first scale: the loud list."""
