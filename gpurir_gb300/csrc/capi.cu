@@ -648,10 +648,10 @@ static int plan_moment(gpurir_sim *s, const std::vector<RoomDesc> &R, Plan &P) {
         P.axis_cap = std::max(P.axis_cap, r.nb[0] + r.nb[1] + r.nb[2]);
         covered += (double)r.n_src * r.n_rcv * std::min<double>(r.n_ism, room_span(r));
     }
-    // Costs in cycles of one SM with two blocks at work (measured): 2.9 per image (the
-    // integer atomics of 32 images take ~90), and per segment the filter, the sums' zeroing
+    // Costs in cycles of one SM with two blocks at work (measured): 2.7 per image (the
+    // integer atomics of 32 images take ~60 and their loads ~15, at 80 % of the pipe), and per segment the filter, the sums' zeroing
     // and their way into the basis, ~8000 at 1024 samples and 16 kHz.
-    const double per_image = 2.9;
+    const double per_image = 2.7;
     auto segment_cost = [&](int T) { return 0.11 * T * P.mom->n_quads + 3000.0; };
     double images = 0.0;
     for (const RoomDesc &r : R)
@@ -673,7 +673,7 @@ static int plan_moment(gpurir_sim *s, const std::vector<RoomDesc> &R, Plan &P) {
     const double fixed = segment_cost(T);
     struct Seg { int lo, hi; double cost; };
     std::vector<std::vector<Seg>> segs(R.size());
-    double total = 0.0, images_cost = 0.0;
+    double total = 0.0, images_cost = 0.0, heaviest = 0.0;
     long busy = 0;   // segments with images
     for (size_t ri = 0; ri < R.size(); ri++) {
         const RoomDesc &r = R[ri];
@@ -686,6 +686,7 @@ static int plan_moment(gpurir_sim *s, const std::vector<RoomDesc> &R, Plan &P) {
                 const double c = per_image * shell_images(r, a - r.H, b + r.H);
                 g.cost += fixed + c;
                 images_cost += c * M;
+                heaviest = std::max(heaviest, c);
                 busy += (long)M;
             }
             total += g.cost * M;
@@ -693,9 +694,27 @@ static int plan_moment(gpurir_sim *s, const std::vector<RoomDesc> &R, Plan &P) {
         }
     }
     // Parts.  Every part of a segment repeats its fixed cost, so a launch that does not fill
-    // the GPU is dealt out to one wave of blocks by images, and in a larger one only segments
-    // of twice a block's share are cut.  Light neighbours go into one item.
-    const double share = total / slots, image_share = images_cost / slots, most = total / (4.0 * slots);
+    // the GPU is dealt out to one wave of blocks, the heaviest part as light as that
+    // allows, and in a larger one only segments of twice a block's share are cut.  Light
+    // neighbours go into one item.
+    const double share = total / slots, most = total / (4.0 * slots);
+    auto most_parts = [&](double images_of) { return std::max(1.0, std::floor(images_of / (per_image * 1024))); };
+    double part_share = images_cost / slots;   // images of the heaviest part
+    if (busy < slots) {
+        double lo = part_share, hi = std::max(heaviest, lo);
+        for (int it = 0; it < 24; it++) {
+            const double mid = 0.5 * (lo + hi);
+            double parts = 0.0;
+            for (size_t ri = 0; ri < R.size(); ri++)
+                for (const Seg &g : segs[ri]) {
+                    const double images_of = g.cost - fixed - 500.0;
+                    if (images_of > 0.0)
+                        parts += (double)R[ri].n_src * R[ri].n_rcv * std::min(std::ceil(images_of / mid), most_parts(images_of));
+                }
+            (parts <= slots ? hi : lo) = mid;
+        }
+        part_share = hi;
+    }
     P.rirs.reserve(M_tot);
     std::vector<IsmItem> work;
     std::vector<std::pair<double, int>> cost;
@@ -707,8 +726,8 @@ static int plan_moment(gpurir_sim *s, const std::vector<RoomDesc> &R, Plan &P) {
         std::vector<Group> items;
         for (const Seg &g : segs[ri]) {
             const double images_of = std::max(g.cost - fixed - 500.0, 0.0);
-            double n = busy < slots ? std::floor(images_of / image_share) : (g.cost > 2.0 * share ? std::ceil(g.cost / share) : 1.0);
-            const int parts = (int)std::max(1.0, std::min(n, images_of / (per_image * 1024)));
+            const double n = busy < slots ? std::ceil(images_of / part_share) : (g.cost > 2.0 * share ? std::ceil(g.cost / share) : 1.0);
+            const int parts = (int)std::max(1.0, std::min(n, most_parts(images_of)));
             if (!items.empty() && parts == 1 && items.back().parts == 1 && items.back().cost + g.cost <= most &&
                 (g.lo - items.back().lo) % T == 0) {
                 items.back().hi = g.hi;
