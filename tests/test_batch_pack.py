@@ -11,7 +11,7 @@ def _rooms():
     return [
         dict(room_sz=[3, 4.1, 2], beta=f(6), pos_src=f(2, 3), pos_rcv=f(5, 3).astype(np.float32), nb_img=[3, 4, 5], Tmax=0.3),
         dict(room_sz=f(3, 1), beta=list(f(6)), pos_src=list(f(3)), pos_rcv=f(3, 2).T[:, [0, 1, 1]].tolist(),
-             nb_img=np.array([6.0, 7.9, 8.0]), Tmax=np.float32(0.2), Tdiff=0.1, mic_pattern="card", orV_rcv=f(9)),
+             nb_img=np.array([6.0, 7.9, 8.0]), Tmax=np.float32(0.2), Tdiff=0.1, mic_pattern="card", orV_rcv=f(6)),
         dict(room_sz=f(1, 3).astype(np.float32), beta=f(2, 3), pos_src=f(12)[::2], pos_rcv=f(1, 1, 3),
              nb_img=np.array([[9], [10], [11]]), Tmax=1, Tdiff=None, spkr_pattern="bidir", orV_src=f(2, 3)[::-1],
              mic_pattern=None, orV_rcv=None),
