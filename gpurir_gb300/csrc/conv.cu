@@ -289,14 +289,8 @@ __device__ __forceinline__ void dft16(float2 (&v)[16]) {
 
 __host__ __device__ constexpr int dr16(int s) { return 4 * (s & 3) + (s >> 2); }
 
-// Twiddles w^r, r = 1..15, of one radix-16 pass (w = W[e]): w, w^2, w^4, w^8 from the
-// table, the others as products of at most three of them (4 loads instead of 15; error
-// within 3 roundings).
-__device__ __forceinline__ void twiddle_powers(const float2 *__restrict__ W, int e, float2 (&t)[16]) {
-    t[1] = __ldg(&W[e]);
-    t[2] = __ldg(&W[2 * e]);
-    t[4] = __ldg(&W[4 * e]);
-    t[8] = __ldg(&W[8 * e]);
+// w^3, w^5, ... of w, w^2, w^4, w^8: products of at most three of them.
+__device__ __forceinline__ void twiddle_products(float2 (&t)[16]) {
     t[3] = cmul(t[1], t[2]);
     t[5] = cmul(t[1], t[4]);
     t[6] = cmul(t[2], t[4]);
@@ -308,6 +302,17 @@ __device__ __forceinline__ void twiddle_powers(const float2 *__restrict__ W, int
     t[13] = cmul(t[5], t[8]);
     t[14] = cmul(t[6], t[8]);
     t[15] = cmul(t[7], t[8]);
+}
+
+// Twiddles w^r, r = 1..15, of one radix-16 pass (w = W[e]): w, w^2, w^4, w^8 from the
+// table, the others as products of at most three of them (4 loads instead of 15; error
+// within 3 roundings).
+__device__ __forceinline__ void twiddle_powers(const float2 *__restrict__ W, int e, float2 (&t)[16]) {
+    t[1] = __ldg(&W[e]);
+    t[2] = __ldg(&W[2 * e]);
+    t[4] = __ldg(&W[4 * e]);
+    t[8] = __ldg(&W[8 * e]);
+    twiddle_products(t);
 }
 
 // One radix-16 Stockham pass at stride Ns for the thread's j (= thread index):
@@ -391,17 +396,55 @@ __device__ __forceinline__ void reg_fft(float2 (&v)[16], float2 *buf, const floa
     __syncthreads();
 }
 
+// Shared-memory twiddles of the row transforms' passes: for each pass of stride Ns the
+// powers 1, 2, 4, 8 of its Ns twiddles, [4][Ns], one pass after the other.  A persistent
+// block copies them once; read from the table in global memory, whose stride of
+// 2M / 16 Ns elements spreads a warp over up to 32 lines, they were 40 % of the load
+// pipe's wavefronts and the longest stall (8192 points, 3200 rows: 244 us, with the tables 215).
+template <int M>
+struct RowTw {
+    static constexpr bool fused = M == 8192;               // radix-2 passes folded into the spectral step
+    static constexpr int head = 4 * 16 + (M >= 4096 ? 4 * 256 : 0);
+    static constexpr int tail = fused ? 4 * (2 + 32 + 512) : 0;
+    static constexpr int bins = fused ? M / 2 : 0;         // W[u], then W[2u], u < M/4: the spectral step's
+};
+template <int M>
+__device__ __forceinline__ void row_twiddles_pass(float2 *tw, int Ns, const float2 *__restrict__ W) {
+    for (int e = threadIdx.x; e < 4 * Ns; e += M / 16) {
+        const int i = e / Ns, k = e - i * Ns;
+        tw[e] = __ldg(&W[(k << i) * ((2 * M) / (Ns * 16))]);
+    }
+}
+template <int M>
+__device__ __forceinline__ void row_twiddles(float2 *tw, const float2 *__restrict__ W) {
+    row_twiddles_pass<M>(tw, 16, W);
+    if (M >= 4096) row_twiddles_pass<M>(tw + 64, 256, W);
+    if (RowTw<M>::fused) {
+        row_twiddles_pass<M>(tw + RowTw<M>::head, 2, W);
+        row_twiddles_pass<M>(tw + RowTw<M>::head + 8, 32, W);
+        row_twiddles_pass<M>(tw + RowTw<M>::head + 136, 512, W);
+        float2 *b = tw + RowTw<M>::head + RowTw<M>::tail;
+        for (int u = threadIdx.x; u < M / 4; u += M / 16) {
+            b[u] = __ldg(&W[u]);
+            b[M / 4 + u] = __ldg(&W[2 * u]);
+        }
+    }
+}
+
 // ROWS transforms at once (rows q at buf + q * pad16(M)): the same passes, barriers
 // and twiddle loads serve every row, and each thread has ROWS independent DFTs in
-// flight per pass.
+// flight per pass.  tw: the pass's twiddles (RowTw).
 template <bool INV, int M, int ROWS>
-__device__ __forceinline__ void pass16_rows(float2 (&v)[ROWS][16], float2 *buf, int j, int Ns,
-                                            const float2 *__restrict__ W) {
+__device__ __forceinline__ void pass16_rows(float2 (&v)[ROWS][16], float2 *buf, int j, int Ns, const float2 *tw) {
     constexpr int BS = M + M / 16;
     const int k = j & (Ns - 1);
     if (Ns > 1) {
         float2 t[16];
-        twiddle_powers(W, k * ((2 * M) / (Ns * 16)), t);
+        t[1] = tw[k];
+        t[2] = tw[Ns + k];
+        t[4] = tw[2 * Ns + k];
+        t[8] = tw[3 * Ns + k];
+        twiddle_products(t);
 #pragma unroll
         for (int r = 1; r < 16; r++) {
             const float2 w = INV ? cconj(t[r]) : t[r];
@@ -419,7 +462,8 @@ __device__ __forceinline__ void pass16_rows(float2 (&v)[ROWS][16], float2 *buf, 
 }
 
 template <bool INV, int M, bool LOADED, int ROWS>
-__device__ __forceinline__ void reg_fft_rows(float2 (&v)[ROWS][16], float2 *buf, const float2 *__restrict__ W) {
+__device__ __forceinline__ void reg_fft_rows(float2 (&v)[ROWS][16], float2 *buf, const float2 *__restrict__ W,
+                                             const float2 *tw) {
     constexpr int T = M / 16, BS = M + M / 16;
     const int j = threadIdx.x;
     if (!LOADED) {
@@ -429,17 +473,17 @@ __device__ __forceinline__ void reg_fft_rows(float2 (&v)[ROWS][16], float2 *buf,
             for (int r = 0; r < 16; r++) v[q][r] = buf[q * BS + pad16(j + r * T)];
         __syncthreads();
     }
-    pass16_rows<INV, M, ROWS>(v, buf, j, 1, W);
+    pass16_rows<INV, M, ROWS>(v, buf, j, 1, tw);
     __syncthreads();
     int Ns = 16;
 #pragma unroll 1
-    for (; Ns * 16 <= M; Ns *= 16) {
+    for (; Ns * 16 <= M; tw += 4 * Ns, Ns *= 16) {
 #pragma unroll
         for (int q = 0; q < ROWS; q++)
 #pragma unroll
             for (int r = 0; r < 16; r++) v[q][r] = buf[q * BS + pad16(j + r * T)];
         __syncthreads();
-        pass16_rows<INV, M, ROWS>(v, buf, j, Ns, W);
+        pass16_rows<INV, M, ROWS>(v, buf, j, Ns, tw);
         __syncthreads();
     }
     if (Ns < M) {   // last pass, radix R = M / Ns in {2, 4, 8}, as in reg_fft
@@ -489,36 +533,36 @@ __device__ __forceinline__ void reg_fft_rows(float2 (&v)[ROWS][16], float2 *buf,
 // Z[k + M/2] = A[k] - W_M^k B[k]); reg_fft_rows_tail runs the radix-16 passes that
 // follow an external first radix-2 pass (Ns = 2, 32, 512, ...).
 template <bool INV, int M, int ROWS>
-__device__ __forceinline__ void reg_fft_rows_head(float2 (&v)[ROWS][16], float2 *buf, const float2 *__restrict__ W) {
+__device__ __forceinline__ void reg_fft_rows_head(float2 (&v)[ROWS][16], float2 *buf, const float2 *tw) {
     constexpr int T = M / 16, BS = M + M / 16;
     const int j = threadIdx.x;
-    pass16_rows<INV, M, ROWS>(v, buf, j, 1, W);   // v loaded by the caller
+    pass16_rows<INV, M, ROWS>(v, buf, j, 1, tw);   // v loaded by the caller
     __syncthreads();
     int Ns = 16;
 #pragma unroll 1
-    for (; Ns * 16 <= M; Ns *= 16) {
+    for (; Ns * 16 <= M; tw += 4 * Ns, Ns *= 16) {
 #pragma unroll
         for (int q = 0; q < ROWS; q++)
 #pragma unroll
             for (int r = 0; r < 16; r++) v[q][r] = buf[q * BS + pad16(j + r * T)];
         __syncthreads();
-        pass16_rows<INV, M, ROWS>(v, buf, j, Ns, W);
+        pass16_rows<INV, M, ROWS>(v, buf, j, Ns, tw);
         __syncthreads();
     }
 }
 
 template <bool INV, int M, int ROWS>
-__device__ __forceinline__ void reg_fft_rows_tail(float2 (&v)[ROWS][16], float2 *buf, const float2 *__restrict__ W) {
+__device__ __forceinline__ void reg_fft_rows_tail(float2 (&v)[ROWS][16], float2 *buf, const float2 *tw) {
     constexpr int T = M / 16, BS = M + M / 16;
     const int j = threadIdx.x;
 #pragma unroll 1
-    for (int Ns = 2; Ns * 16 <= M; Ns *= 16) {
+    for (int Ns = 2; Ns * 16 <= M; tw += 4 * Ns, Ns *= 16) {
 #pragma unroll
         for (int q = 0; q < ROWS; q++)
 #pragma unroll
             for (int r = 0; r < 16; r++) v[q][r] = buf[q * BS + pad16(j + r * T)];
         __syncthreads();
-        pass16_rows<INV, M, ROWS>(v, buf, j, Ns, W);
+        pass16_rows<INV, M, ROWS>(v, buf, j, Ns, tw);
         __syncthreads();
     }
 }
@@ -605,11 +649,29 @@ __global__ void __launch_bounds__(M / 16, 16384 / M) segment_spectra_reg_kernel(
 // inputs); the values wait in v, free between the transforms.
 template <int M, int ROWS>
 __device__ __forceinline__ void conv_spectral_fused(float2 (&v)[ROWS][16], float2 *buf, const float2 *__restrict__ W,
-                                                    const float2 *__restrict__ Sg, int pr0, int nq, int R) {
+                                                    const float2 *tw, const float2 *__restrict__ Sg, int pr0, int nq,
+                                                    int R) {
     constexpr int T = M / 16, BS = M + M / 16, H = M / 2, Q = M / 4;
     static_assert(Q == 4 * T, "four units per thread");
     const int j = threadIdx.x;
-    reg_fft_rows_head<false, M, ROWS>(v, buf, W);
+    const float2 *wb = tw + RowTw<M>::head + RowTw<M>::tail;
+    reg_fft_rows_head<false, M, ROWS>(v, buf, tw);
+    // segment spectrum at the thread's bins k, M - k, k', M - k' (rows of one point share it):
+    // asked for before the barrier
+    float2 s4[4][4];
+    const int p0 = pr0 / R;
+    auto spectrum = [&](int p) {
+        const float2 *sp = Sg + (size_t)p * (M + 1);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int k = j + i * T, kp = H - k;
+            s4[i][0] = __ldg(&sp[k]);
+            s4[i][1] = __ldg(&sp[M - k]);
+            s4[i][2] = __ldg(&sp[kp]);
+            s4[i][3] = __ldg(&sp[M - kp]);
+        }
+    };
+    spectrum(p0);
     float2 e[ROWS][2];   // unit M/4 (thread 0 only): Z[M/4], Z[3M/4]
 #pragma unroll
     for (int q = 0; q < ROWS; q++) {
@@ -618,13 +680,14 @@ __device__ __forceinline__ void conv_spectral_fused(float2 (&v)[ROWS][16], float
         for (int i = 0; i < 4; i++) {
             const int u = j + i * T;
             if (u == 0) {   // bins 0 and M/2: Z[0] = A[0] + B[0], Z[M/2] = A[0] - B[0]
-                float2 a0 = bq[pad16(0)], a1 = cmul(bq[pad16(H)], __ldg(&W[0]));
+                float2 a0 = bq[pad16(0)], a1 = cmul(bq[pad16(H)], wb[0]);
                 v[q][4 * i] = cadd(a0, a1);
                 v[q][4 * i + 1] = csub(a0, a1);
             } else {
                 const int k = u, kp = H - u;
-                const float2 ak = bq[pad16(k)], bk = cmul(bq[pad16(k + H)], __ldg(&W[2 * k]));
-                const float2 ap = bq[pad16(kp)], bp = cmul(bq[pad16(kp + H)], __ldg(&W[2 * kp]));
+                const float2 w = wb[Q + u], wp = make_float2(-w.x, w.y);   // W[2k], W[2k']
+                const float2 ak = bq[pad16(k)], bk = cmul(bq[pad16(k + H)], w);
+                const float2 ap = bq[pad16(kp)], bp = cmul(bq[pad16(kp + H)], wp);
                 v[q][4 * i] = cadd(ak, bk);        // Z[k]
                 v[q][4 * i + 1] = csub(ak, bk);    // Z[k + M/2] = Z[M - k']
                 v[q][4 * i + 2] = cadd(ap, bp);    // Z[k']
@@ -642,23 +705,25 @@ __device__ __forceinline__ void conv_spectral_fused(float2 (&v)[ROWS][16], float
     for (int q = 0; q < ROWS; q++) {
         if (q >= nq) break;
         float2 *bq = buf + q * BS;
-        const float2 *sp = Sg + (size_t)((pr0 + q) / R) * (M + 1);
+        const int p = (pr0 + q) / R;
+        const float2 *sp = Sg + (size_t)p * (M + 1);
+        if (q > 0 && p != (pr0 + q - 1) / R) spectrum(p);
 #pragma unroll
         for (int i = 0; i < 4; i++) {
             const int u = j + i * T;
             if (u == 0) {
                 float2 y0, yM, yh, yh2;
-                conv_bin_pair(v[q][0], v[q][0], __ldg(&W[0]), __ldg(&sp[0]), __ldg(&sp[M]), y0, yM);
-                conv_bin_pair(v[q][1], v[q][1], __ldg(&W[H]), __ldg(&sp[H]), __ldg(&sp[H]), yh, yh2);
+                conv_bin_pair(v[q][0], v[q][0], wb[0], s4[i][0], s4[i][1], y0, yM);
+                conv_bin_pair(v[q][1], v[q][1], __ldg(&W[H]), s4[i][2], s4[i][3], yh, yh2);
                 bq[pad16(0)] = cadd(y0, yh);
                 bq[pad16(1)] = csub(y0, yh);
             } else {
                 const int k = u, kp = H - u;
                 float2 yk, ymk, ykp, ymkp;
                 // pair (k, M - k): Z[k], Z[M - k] = Z[k' + M/2]; pair (k', M - k'): Z[k'], Z[k + M/2]
-                conv_bin_pair(v[q][4 * i], v[q][4 * i + 3], __ldg(&W[k]), __ldg(&sp[k]), __ldg(&sp[M - k]), yk, ymk);
-                conv_bin_pair(v[q][4 * i + 2], v[q][4 * i + 1], __ldg(&W[kp]), __ldg(&sp[kp]), __ldg(&sp[M - kp]),
-                              ykp, ymkp);
+                const float2 w = wb[u], wp = make_float2(-w.y, -w.x);   // W[k], W[k']
+                conv_bin_pair(v[q][4 * i], v[q][4 * i + 3], w, s4[i][0], s4[i][1], yk, ymk);
+                conv_bin_pair(v[q][4 * i + 2], v[q][4 * i + 1], wp, s4[i][2], s4[i][3], ykp, ymkp);
                 // the inverse's first radix-2 pass: out[2j] = Y'[j] + Y'[j + M/2], out[2j + 1] = difference
                 bq[pad16(2 * k)] = cadd(yk, ymkp);        // Y'[k + M/2] = Y'[M - k']
                 bq[pad16(2 * k + 1)] = csub(yk, ymkp);
@@ -674,7 +739,7 @@ __device__ __forceinline__ void conv_spectral_fused(float2 (&v)[ROWS][16], float
         }
     }
     __syncthreads();
-    reg_fft_rows_tail<true, M, ROWS>(v, buf, W);
+    reg_fft_rows_tail<true, M, ROWS>(v, buf, tw + RowTw<M>::head);
 }
 
 template <int M, int ROWS>
@@ -684,6 +749,8 @@ __global__ void __launch_bounds__(M / 16, (16384 / M / ROWS > 0 ? 16384 / M / RO
     constexpr int T = M / 16, BS = M + M / 16;
     extern __shared__ __align__(16) float2 sm[];
     float2 *buf = sm;   // ROWS buffers of pad16(M) elements
+    float2 *tw = sm + ROWS * BS;
+    row_twiddles<M>(tw, W);   // (the first pass needs none: its barrier is before their first use)
     const int j = threadIdx.x;
     const int n_out = S + L - 1;
     float2 v[ROWS][16];
@@ -711,9 +778,9 @@ __global__ void __launch_bounds__(M / 16, (16384 / M / ROWS > 0 ? 16384 / M / RO
             }
         }
         if constexpr (M == 8192) {
-            conv_spectral_fused<M, ROWS>(v, buf, W, Sg, pr0, nq, R);
+            conv_spectral_fused<M, ROWS>(v, buf, W, tw, Sg, pr0, nq, R);
         } else {
-        reg_fft_rows<false, M, true, ROWS>(v, buf, W);
+        reg_fft_rows<false, M, true, ROWS>(v, buf, W, tw);
         // spectrum of the RIR at k and M - k, times the segment's spectrum, repacked
         // for the inverse real FFT (same algebra as rir_conv_kernel).  The thread's k are
         // j + i T; their twiddles and segment spectra are loaded four k at a time before
@@ -757,7 +824,7 @@ __global__ void __launch_bounds__(M / 16, (16384 / M / ROWS > 0 ? 16384 / M / RO
             }
         }
         __syncthreads();
-        reg_fft_rows<true, M, false, ROWS>(v, buf, W);
+        reg_fft_rows<true, M, false, ROWS>(v, buf, W, tw);
         }
         for (int q = 0; q < nq; q++) {
             const float2 *bq = buf + q * BS;
@@ -785,7 +852,7 @@ constexpr int kTuneTrajBlocksKnob = 3; // TuneKnob::kTuneTrajBlocksPerSm
 template <int M, int ROWS>
 static cudaError_t launch_reg_conv_rows(const float *rir, int P, int R, int L, int S, const float2 *W,
                                         const float2 *Sg, float *out, long out_ld, cudaStream_t st) {
-    const size_t smem = (size_t)ROWS * (M + M / 16) * sizeof(float2);
+    const size_t smem = ((size_t)ROWS * (M + M / 16) + RowTw<M>::head + RowTw<M>::tail + RowTw<M>::bins) * sizeof(float2);
     static int blocks = -1;
     if (blocks < 0) {
         cudaError_t e = cudaFuncSetAttribute(rir_conv_reg_kernel<M, ROWS>,
@@ -1015,17 +1082,7 @@ __device__ __forceinline__ void blk_powers(const float2 *tw, float2 (&t)[16]) {
     t[2] = tw[T + j];
     t[4] = tw[2 * T + j];
     t[8] = tw[3 * T + j];
-    t[3] = cmul(t[1], t[2]);
-    t[5] = cmul(t[1], t[4]);
-    t[6] = cmul(t[2], t[4]);
-    t[7] = cmul(t[3], t[4]);
-    t[9] = cmul(t[1], t[8]);
-    t[10] = cmul(t[2], t[8]);
-    t[11] = cmul(t[3], t[8]);
-    t[12] = cmul(t[4], t[8]);
-    t[13] = cmul(t[5], t[8]);
-    t[14] = cmul(t[6], t[8]);
-    t[15] = cmul(t[7], t[8]);
+    twiddle_products(t);
 }
 
 // Forward transform: v[r] = z[j + 128 r] in, v[8 g + s] = Z[j + 128 g + 256 s] out.
