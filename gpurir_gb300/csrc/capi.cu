@@ -440,6 +440,7 @@ struct Plan {
     const MomBasis *mom = nullptr;
     int mom_T = 0;                // longest segment
     int mom_win = 0;              // shortest last segment of an item
+    int mom_threads = 0;          // shape of its blocks
     size_t mom_smem = 0;
     std::vector<IsmItem> items;
     std::vector<IsmItem> rirs;
@@ -648,73 +649,117 @@ static int plan_moment(gpurir_sim *s, const std::vector<RoomDesc> &R, Plan &P) {
         P.axis_cap = std::max(P.axis_cap, r.nb[0] + r.nb[1] + r.nb[2]);
         covered += (double)r.n_src * r.n_rcv * std::min<double>(r.n_ism, room_span(r));
     }
-    // Costs in cycles of one SM with two blocks at work (measured): 2.7 per image (the
-    // integer atomics of 32 images take ~60 and their loads ~15, at 80 % of the pipe), and per segment the filter, the sums' zeroing
-    // and their way into the basis, ~8000 at 1024 samples and 16 kHz.
-    const double per_image = 2.7;
-    auto segment_cost = [&](int T) { return 0.11 * T * P.mom->n_quads + 3000.0; };
-    double images = 0.0;
-    for (const RoomDesc &r : R)
-        images += (double)r.n_src * r.n_rcv * shell_images(r, 0.0, std::min<double>(r.n_ism, room_span(r)));
-    // Long segments spend less on what neighbours share (their taps' reach, 12 % of the images at
-    // 1024 samples and 16 kHz, 25 % at 512); short ones give a small launch more items.  A
-    // segment of many images can be dealt to several items instead.
-    const long slots = 2L * s->num_sms;   // (not of a tuned grid: the items fix the results' bits)
-    P.mom_T = 1024;
-    if (covered / 1024 < slots && images * per_image < 2.0 * covered / 1024 * segment_cost(1024)) P.mom_T = 512;
-    if (moment_cells(P.mom_T, *P.mom) > kMomCells) return fail(GPURIR_ERR_UNSUPPORTED, "window too long");   // (not reached)
-    P.mom_smem = moment_smem_bytes(P.axis_cap, *P.mom);
-    int bps = moment_blocks_per_sm(P.mom_smem);
+    // Costs in cycles of one SM with its blocks at work (measured, two large blocks): 2.8 per
+    // image (the integer atomics of 32 images take ~60 and their loads ~15, at 80 % of the
+    // pipe), and per segment the filter, the sums' zeroing and their way into the basis, ~10000
+    // at 1024 samples and 16 kHz.  Three small blocks take 0.8 of the latter and as much per image.
+    const double per_image = 2.8, per_item = 500.0, per_launch = 10000.0;
+    struct Seg { int lo, hi; float images, rest, most; double n; };   // cost of its images, other cost, most parts, RIRs
+    typedef std::vector<std::vector<Seg>> Segs;
+    const int win = (int)std::ceil(0.01 * R[0].fs) + 2;
+    auto cut_segments = [&](int T) {   // as the kernel cuts an item's samples
+        Segs segs(R.size());
+        const double fixed = 0.14 * T * P.mom->n_quads + 3500.0;
+        const int least = win <= T - 4 ? win : 0;
+        for (size_t ri = 0; ri < R.size(); ri++) {
+            const RoomDesc &r = R[ri];
+            const double span = room_span(r);
+            for (int a = 0, b; a < r.n_ism; a = b) {
+                b = std::min(a + T, r.n_ism);
+                if (b < r.n_ism && r.n_ism - b < least) b = (r.n_ism - least) & ~3;
+                Seg g = {a, b, 0.0f, (float)per_item, 1.0f, (double)r.n_src * r.n_rcv};
+                if (a < span) {
+                    const double n = shell_images(r, a - r.H, b + r.H);
+                    g.images = (float)(per_image * n);
+                    g.rest += (float)fixed;
+                    g.most = (float)std::max(1.0, std::floor(n / 1024.0));   // a part holds 1024 images at least
+                }
+                segs[ri].push_back(g);
+            }
+        }
+        return segs;
+    };
+    auto parts_of = [](const Seg &g, float limit) {
+        return std::max(1.0f, std::min((float)(int)(g.images / limit + 0.9999f), g.most));
+    };
+    // Time of a launch whose segments are cut into parts of at most `limit` (cost of images), in
+    // cost per slot: its heaviest item if one wave holds them all, else the mean load and, for
+    // the uneven end, half a mean item; the launches that add parts up.
+    auto judge = [&](const Segs &segs, double slots, float rest, float limit, double &n) {
+        double total = 0.0;
+        float worst = 0.0f, parts = 1.0f;
+        n = 0.0;
+        for (const std::vector<Seg> &room : segs)
+            for (const Seg &g : room) {
+                const float p = parts_of(g, limit), c = g.images / p + rest * g.rest;
+                total += g.n * (p * c);
+                if (g.rest > (float)per_item) n += g.n * p;
+                worst = std::max(worst, c);
+                parts = std::max(parts, p);
+            }
+        return (n <= slots ? worst : std::max<double>(worst, total / slots) + 0.5 * total / n) + (parts > 1.0f ? per_launch : 0.0);
+    };
+    // The shape of the blocks, the segments' length and the size of parts by the least time of
+    // these.  Long segments spend less on what neighbours share (their taps' reach, 12 % of the
+    // images at 1024 samples and 16 kHz, 25 % at 512); short ones give a small launch more items.
+    // Every part of a segment repeats its fixed cost.  (Not of a tuned grid: the items fix the
+    // results' bits.)
+    P.mom_T = 0;
+    double best = INFINITY;
+    float part_limit = INFINITY;
+    Segs segs;
+    for (int T : {1024, 512}) {
+        if (T == 512 && covered / 1024 > 2.0 * s->num_sms && moment_cells(1024, *P.mom) <= kMomSmallCells) break;
+        Segs with = cut_segments(T);
+        double images = 0.0;
+        for (const std::vector<Seg> &room : with)
+            for (const Seg &g : room) images += g.n * g.images;
+        for (int threads : {kMomLarge, kMomSmall}) {
+            const double blocks = threads == kMomSmall ? 3.0 : 2.0, slots = blocks * s->num_sms;
+            const float rest = threads == kMomSmall ? 0.8f : 1.0f;
+            if (moment_cells(T, *P.mom) > (threads == kMomSmall ? kMomSmallCells : kMomCells)) continue;
+            // (tables in global memory want the L1 that three blocks take: 48 rooms 278 us, with three 329)
+            if (threads == kMomSmall && (P.axis_cap > kMomTabSmem ||
+                                         moment_blocks_per_sm(threads, moment_smem_bytes(threads, P.axis_cap, *P.mom)) < 3)) continue;
+            auto consider = [&](float limit) {
+                double n;
+                const double t = blocks * judge(with, slots, rest, limit, n);
+                if (t < best) {
+                    best = t;
+                    part_limit = limit;
+                    P.mom_T = T;
+                    P.mom_threads = threads;
+                }
+                return n;
+            };
+            const double share = std::max(images / slots, 1.0);
+            const double n = consider(INFINITY);
+            for (double f = 2.0; f > 0.1; f *= 0.5) consider((float)(f * share));
+            if (n < slots) {   // one wave: the smallest limit it holds
+                double lo = share, hi = images;
+                for (int it = 0; it < 12 && hi > 1.03 * lo; it++) {
+                    const double mid = std::sqrt(lo * hi);
+                    double items;
+                    judge(with, slots, rest, (float)mid, items);
+                    (items <= slots ? hi : lo) = mid;
+                }
+                consider((float)hi);
+            }
+        }
+        if (P.mom_T == T) segs = std::move(with);
+    }
+    if (segs.empty()) return fail(GPURIR_ERR_UNSUPPORTED, "window too long");   // (use_moments)
+    const int T = P.mom_T;
+    P.mom_win = win <= T - 4 ? win : 0;
+    P.mom_smem = moment_smem_bytes(P.mom_threads, P.axis_cap, *P.mom);
+    int bps = moment_blocks_per_sm(P.mom_threads, P.mom_smem);
     if (bps < 1) return fail(GPURIR_ERR_CUDA, "ISM kernel does not fit on an SM");
     if (tuning(1) > 0) bps = std::min(bps, tuning(1));   // ism_blocks_per_sm (tuning.cu)
-    const int T = P.mom_T;
-    const int win = (int)std::ceil(0.01 * R[0].fs) + 2;
-    P.mom_win = win <= T - 4 ? win : 0;
-    const double fixed = segment_cost(T);
-    struct Seg { int lo, hi; double cost; };
-    std::vector<std::vector<Seg>> segs(R.size());
-    double total = 0.0, images_cost = 0.0, heaviest = 0.0;
-    long busy = 0;   // segments with images
-    for (size_t ri = 0; ri < R.size(); ri++) {
-        const RoomDesc &r = R[ri];
-        const double span = room_span(r), M = (double)r.n_src * r.n_rcv;
-        for (int a = 0, b; a < r.n_ism; a = b) {   // as the kernel cuts an item's samples
-            b = std::min(a + T, r.n_ism);
-            if (b < r.n_ism && r.n_ism - b < P.mom_win) b = (r.n_ism - P.mom_win) & ~3;
-            Seg g = {a, b, 500.0};
-            if (a < span) {
-                const double c = per_image * shell_images(r, a - r.H, b + r.H);
-                g.cost += fixed + c;
-                images_cost += c * M;
-                heaviest = std::max(heaviest, c);
-                busy += (long)M;
-            }
-            total += g.cost * M;
-            segs[ri].push_back(g);
-        }
-    }
-    // Parts.  Every part of a segment repeats its fixed cost, so a launch that does not fill
-    // the GPU is dealt out to one wave of blocks, the heaviest part as light as that
-    // allows, and in a larger one only segments of twice a block's share are cut.  Light
-    // neighbours go into one item.
-    const double share = total / slots, most = total / (4.0 * slots);
-    auto most_parts = [&](double images_of) { return std::max(1.0, std::floor(images_of / (per_image * 1024))); };
-    double part_share = images_cost / slots;   // images of the heaviest part
-    if (busy < slots) {
-        double lo = part_share, hi = std::max(heaviest, lo);
-        for (int it = 0; it < 24; it++) {
-            const double mid = 0.5 * (lo + hi);
-            double parts = 0.0;
-            for (size_t ri = 0; ri < R.size(); ri++)
-                for (const Seg &g : segs[ri]) {
-                    const double images_of = g.cost - fixed - 500.0;
-                    if (images_of > 0.0)
-                        parts += (double)R[ri].n_src * R[ri].n_rcv * std::min(std::ceil(images_of / mid), most_parts(images_of));
-                }
-            (parts <= slots ? hi : lo) = mid;
-        }
-        part_share = hi;
-    }
+    // light neighbours go into one item
+    double total = 0.0;
+    for (const std::vector<Seg> &room : segs)
+        for (const Seg &g : room) total += g.n * (g.images + g.rest);
+    const double most = total / (4.0 * (P.mom_threads == kMomSmall ? 3.0 : 2.0) * s->num_sms);
     P.rirs.reserve(M_tot);
     std::vector<IsmItem> work;
     std::vector<std::pair<double, int>> cost;
@@ -725,15 +770,14 @@ static int plan_moment(gpurir_sim *s, const std::vector<RoomDesc> &R, Plan &P) {
         struct Group { int lo, hi, parts; double cost; };
         std::vector<Group> items;
         for (const Seg &g : segs[ri]) {
-            const double images_of = std::max(g.cost - fixed - 500.0, 0.0);
-            const double n = busy < slots ? std::ceil(images_of / part_share) : (g.cost > 2.0 * share ? std::ceil(g.cost / share) : 1.0);
-            const int parts = (int)std::max(1.0, std::min(n, most_parts(images_of)));
-            if (!items.empty() && parts == 1 && items.back().parts == 1 && items.back().cost + g.cost <= most &&
+            const int parts = (int)parts_of(g, part_limit);
+            const double cost_of = g.images + g.rest;
+            if (!items.empty() && parts == 1 && items.back().parts == 1 && items.back().cost + cost_of <= most &&
                 (g.lo - items.back().lo) % T == 0) {
                 items.back().hi = g.hi;
-                items.back().cost += g.cost;
+                items.back().cost += cost_of;
             } else {
-                items.push_back({g.lo, g.hi, parts, g.cost});
+                items.push_back({g.lo, g.hi, parts, cost_of});
             }
         }
         const int last = items.empty() ? 0 : segs[ri].back().hi - segs[ri].back().lo;
@@ -938,12 +982,11 @@ static int enqueue_kernels(gpurir_sim *s, const Plan &P, const char *d, const La
         m.coef = reinterpret_cast<const float2 *>(d + L.o_coef);
         memcpy(m.run, P.mom->run, sizeof(m.run));
         m.n_quads = P.mom->n_quads;
-        memcpy(m.cut1, P.mom->cut1, sizeof(m.cut1));
-        memcpy(m.cut2, P.mom->cut2, sizeof(m.cut2));
+        memcpy(m.cut, P.mom->cut[P.mom_threads == kMomSmall], sizeof(m.cut));
         memcpy(m.S, P.mom->S, sizeof(m.S));
         m.seed = ta.seed; m.offset = ta.offset; m.offset_ptr = ta.offset_ptr;
         m.noise_kind = ta.noise_kind; m.env_out = ta.env_out; m.fuse_tail = ta.fuse; m.tail_pre = ta.pre;
-        CK(moment_launch(m, P.mom_smem, P.grid, st));
+        CK(moment_launch(m, P.mom_threads, P.mom_smem, P.grid, st));
     } else if (P.grid > 0)
         CK(ism_forward_launch(P.tpl, drooms, reinterpret_cast<const IsmItem *>(d + L.o_items),
                               (int)P.items.size(), dps, dpr, dos, dor, dout, work_counter,

@@ -54,13 +54,23 @@
 
 namespace gpurir {
 
-constexpr int kMThreads = 384;
-constexpr int kMWarps = kMThreads / 32;
-static_assert(kMWarps == kMomWarps, "");
-constexpr int kMRows = kMThreads;              // image rows per batch
-constexpr int kMStride = kMomCells;            // cells of one array (a constant: offsets are immediates)
-constexpr int kMGroups = 2048;                 // groups of 32 images per batch of rows
-constexpr int kMTwo = 5;                       // pairs of moments with two integers
+// The two shapes of a block: threads, blocks per SM, cells of one array (a constant, so that
+// offsets are immediates), groups of 32 images per batch of rows.  A block's phases (image
+// atomics, filter, output) wait for one another; three small blocks per SM overlap better
+// than two large ones.  128 rooms: 675 us with two, TIMES with three; 8 x 1024 array 370 and TIMES.  The
+// large one is for windows whose cells three blocks cannot hold and for launches of few
+// segments, where each item's fixed cost counts (plan_moment).
+template <int THREADS>
+struct MomCfg {
+    static constexpr int threads = THREADS, warps = THREADS / 32, rows = THREADS;   // rows: image rows per batch
+    static constexpr int blocks = THREADS == kMomSmall ? 3 : 2;
+    static constexpr int stride = THREADS == kMomSmall ? kMomSmallCells : kMomCells;
+    static constexpr int groups = THREADS == kMomSmall ? 1024 : 2048;
+    static constexpr int cells = (stride + THREADS - 1) / THREADS;                  // of one thread
+    static_assert(kPowerThreads > THREADS && kPowerThreads <= 2 * THREADS,
+                  "the fused tail sums the window power in the tail kernel's order");
+};
+constexpr int kMTwo = 4;                       // pairs of moments with two integers
 constexpr int kMSums = 4 * kMTwo + 2 * (kMPairs - kMTwo) + 1;   // integers per cell, the last one the count
 // Packed sums, for cells of fewer than 7/8 2^h images (h <= 9).  Amplitudes span 2^21 steps.
 // T0..T7: two words of steps and, shared by a pair, one with what the rounding left, 16 bits
@@ -69,11 +79,8 @@ constexpr int kMPTwo = 4, kMPSums = 3 * kMPTwo + 2 + 3;
 constexpr int kMPSpan = 21, kMPCount = 10, kMPMinBits = 6, kMPMaxBits = 9;
 static_assert(kMPairs == 7, "the packed words are laid out for fourteen moments");
 constexpr int kMLoud = 32;                     // images of a segment above the bound of its scale
-constexpr int kMTabSmem = 256;                 // per-axis entries of a launch held in shared memory
 constexpr float kMMagic = 12582912.0f;         // 1.5 2^23
 constexpr int kMMagicBits = 0x4b400000;
-static_assert(kPowerThreads > kMThreads && kPowerThreads <= 2 * kMThreads,
-              "the fused tail sums the window power in the tail kernel's order");
 
 // Cell b of a basis pair: 16-byte chunks of two cells, rotated within groups of four so
 // that 16-byte loads of lanes eight cells apart fall on distinct banks.
@@ -94,12 +101,12 @@ constexpr int kItemWords = sizeof(IsmItem) / 4, kRoomWords = offsetof(RoomDesc, 
 static_assert(kItemWords <= 32 && kRoomWords <= 64 && kRoomWords > 32, "copied by one warp in one and two loads");
 
 struct MomSmem {
-    int *sum;                 // [kMSums][kMStride] moments as integers, and images, per cell;
-                              // then [kMBasis][kMStride] float2 and, after those, the filter's parts
+    int *sum;                 // [kMSums][stride] moments as integers, and images, per cell;
+                              // then [kMBasis][stride] float2 and, after those, the filter's parts
     float2 *coef;             // [8 * quads]: four taps x two output phases
-    float4 *rows;             // [kMRows] rho^2 hi, lo, attenuation, m0 | m1 << 16
-    int2 *range;              // [kMRows] first image, za | na << 9 | zb << 18
-    unsigned short *group;    // [kMGroups] row of a group's first image
+    float4 *rows;             // [rows] rho^2 hi, lo, attenuation, m0 | m1 << 16
+    int2 *range;              // [rows] first image, za | na << 9 | zb << 18
+    unsigned short *group;    // [groups] row of a group's first image
     float4 *loud;             // [kMLoud] a, u, cell
     MomCtx *ctx;              // [2]
     int *red;                 // scan scratch [32], control words [16]
@@ -109,19 +116,20 @@ struct MomSmem {
 __host__ __device__ inline size_t mom_align16(size_t x) { return (x + 15) & ~(size_t)15; }
 
 // Byte offsets of the arrays of MomSmem, in its order; returns the total.
+template <class Cfg>
 __host__ __device__ inline size_t mom_layout(int n_quads, int axis_cap, size_t o[9]) {
-    const size_t sums = (size_t)kMSums * kMStride * sizeof(int);
-    const size_t filt = (size_t)kMBasis * kMStride * sizeof(float2) + (size_t)kMWarps * 512 * sizeof(float);
+    const size_t sums = (size_t)kMSums * Cfg::stride * sizeof(int);
+    const size_t filt = (size_t)kMBasis * Cfg::stride * sizeof(float2) + (size_t)Cfg::warps * 512 * sizeof(float);
     size_t b = 0;
     o[0] = b; b = mom_align16(b + (sums > filt ? sums : filt));
     o[1] = b; b = mom_align16(b + (size_t)n_quads * 8 * sizeof(float2));
-    o[2] = b; b = b + kMRows * sizeof(float4);
-    o[3] = b; b = b + kMRows * sizeof(int2);
-    o[4] = b; b = b + kMGroups * sizeof(unsigned short);
+    o[2] = b; b = b + Cfg::rows * sizeof(float4);
+    o[3] = b; b = b + Cfg::rows * sizeof(int2);
+    o[4] = b; b = b + Cfg::groups * sizeof(unsigned short);
     o[5] = b; b = b + kMLoud * sizeof(float4);
     o[6] = b; b = mom_align16(b + 2 * sizeof(MomCtx));
     o[7] = b; b = mom_align16(b + 48 * sizeof(int));
-    o[8] = b; b += axis_cap <= kMTabSmem ? 2 * (size_t)axis_cap * sizeof(float4) : 0;
+    o[8] = b; b += axis_cap <= kMomTabSmem ? 2 * (size_t)axis_cap * sizeof(float4) : 0;
     return b;
 }
 
@@ -133,6 +141,7 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
 
 // Exclusive block scan of one int per thread; `tot` is the block's sum.  red: 32 ints
 // (two calls in a row use different halves of the scratch, so one barrier each).
+template <int WARPS>
 __device__ __forceinline__ int block_scan(int v, int *red, int &tot) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int x = v;
@@ -143,13 +152,13 @@ __device__ __forceinline__ int block_scan(int v, int *red, int &tot) {
     }
     if (lane == 31) red[warp] = x;
     __syncthreads();
-    int w = lane < kMWarps ? red[lane] : 0;
+    int w = lane < WARPS ? red[lane] : 0;
 #pragma unroll
-    for (int o = 1; o < kMWarps; o <<= 1) {
+    for (int o = 1; o < WARPS; o <<= 1) {
         const int y = __shfl_up_sync(0xffffffffu, w, o);
         if (lane >= o) w += y;
     }
-    tot = __shfl_sync(0xffffffffu, w, kMWarps - 1);
+    tot = __shfl_sync(0xffffffffu, w, WARPS - 1);
     const int before = __shfl_sync(0xffffffffu, w, warp > 0 ? warp - 1 : 0);
     return x - v + (warp > 0 ? before : 0);
 }
@@ -292,11 +301,12 @@ __device__ __forceinline__ void ctx_finish(MomCtx &c, const MomLaunch &P, int id
 // Per-axis image terms of one item (as ism_forward.cu tabulates them): {v^2 hi, v^2 lo, v,
 // attenuation} for m < N0, then N1, then N2 entries.  Wall powers come from the room in
 // global memory, everything else from the item's context.
+template <int THREADS>
 __device__ __forceinline__ void axis_tables(const MomLaunch &P, MomCtx &c, float4 *tab, int tid) {
     const RoomDesc &R = *reinterpret_cast<const RoomDesc *>(c.room);
     const RoomDesc &G = P.rooms[c.it.room];
     const int N0 = R.nb[0], N1 = R.nb[1], N2 = R.nb[2];
-    for (int e = tid; e < N0 + N1 + N2; e += kMThreads) {
+    for (int e = tid; e < N0 + N1 + N2; e += THREADS) {
         const int a = e < N0 ? 0 : (e < N0 + N1 ? 1 : 2);
         const int m = e - (a == 0 ? 0 : (a == 1 ? N0 : N0 + N1));
         int ca, fa;
@@ -362,12 +372,15 @@ __device__ __noinline__ void add_loud(float2 (&A)[kMPairs], const float4 *loud, 
     }
 }
 
-__global__ void __launch_bounds__(kMThreads, 2) ism_moment_kernel(const __grid_constant__ MomLaunch P) {
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS, MomCfg<THREADS>::blocks) ism_moment_kernel(const __grid_constant__ MomLaunch P) {
+    using Cfg = MomCfg<THREADS>;
+    constexpr int kMThreads = THREADS, kMWarps = Cfg::warps, kMStride = Cfg::stride;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     MomSmem s;
     {
         size_t o[9];
-        mom_layout(P.n_quads, P.axis_cap, o);
+        mom_layout<Cfg>(P.n_quads, P.axis_cap, o);
         s.sum = reinterpret_cast<int *>(smem_raw + o[0]);
         s.coef = reinterpret_cast<float2 *>(smem_raw + o[1]);
         s.rows = reinterpret_cast<float4 *>(smem_raw + o[2]);
@@ -376,7 +389,7 @@ __global__ void __launch_bounds__(kMThreads, 2) ism_moment_kernel(const __grid_c
         s.loud = reinterpret_cast<float4 *>(smem_raw + o[5]);
         s.ctx = reinterpret_cast<MomCtx *>(smem_raw + o[6]);
         s.red = reinterpret_cast<int *>(smem_raw + o[7]);
-        s.tab = P.axis_cap <= kMTabSmem ? reinterpret_cast<float4 *>(smem_raw + o[8])
+        s.tab = P.axis_cap <= kMomTabSmem ? reinterpret_cast<float4 *>(smem_raw + o[8])
                                         : P.axis_tab + (size_t)(2 * blockIdx.x) * P.axis_cap;
     }
     float2 *basis = reinterpret_cast<float2 *>(s.sum);                 // [kMBasis][kMStride]
@@ -397,7 +410,7 @@ __global__ void __launch_bounds__(kMThreads, 2) ism_moment_kernel(const __grid_c
         ctx_finish(s.ctx[0], P, next, lane);
     }
     __syncthreads();
-    if (s.ctx[0].valid) axis_tables(P, s.ctx[0], s.tab, tid);
+    if (s.ctx[0].valid) axis_tables<THREADS>(P, s.ctx[0], s.tab, tid);
 
     for (int par = 0;; par ^= 1) {
         const MomCtx &C = s.ctx[par];
@@ -446,7 +459,7 @@ __global__ void __launch_bounds__(kMThreads, 2) ism_moment_kernel(const __grid_c
                 my_rows = n_box > C.it.i_lo ? (n_box - C.it.i_lo + C.it.i_hi - 1) / C.it.i_hi : 0;
             }
             const float rW1 = 1.0f / (float)max(W1, 1);
-            const int batch = min(kMRows, 32 * kMGroups / N2);   // rows at once: their images fill the groups at most
+            const int batch = min(Cfg::rows, 32 * Cfg::groups / N2);   // rows at once: their images fill the groups at most
             // mean images per cell at the segment's end: a room's volume holds one; cells with few
             // have packed sums
             const float mean = 25.14f * d_hi * d_hi * C.inv_k * C.inv_L[0] * C.inv_L[1] * inv_L2 / (float)C.it.i_hi;
@@ -522,7 +535,7 @@ __global__ void __launch_bounds__(kMThreads, 2) ism_moment_kernel(const __grid_c
                     }
                     const int na = ya - za, mine = na + (yb - zb);
                     int total;
-                    const int scan = block_scan(mine | (mine > 0 ? 1 << 20 : 0), s.red, total);
+                    const int scan = block_scan<kMWarps>(mine | (mine > 0 ? 1 << 20 : 0), s.red, total);
                     const int off = scan & 0xfffff, my_row = scan >> 20;   // images and rows with images before mine
                     if (mine > 0) {
                         s.rows[my_row] = row;
@@ -649,9 +662,9 @@ __global__ void __launch_bounds__(kMThreads, 2) ism_moment_kernel(const __grid_c
             act = ctl[1] >= 0 ? min((ctl[1] >> 8) + 1, tiles) : 0;
             // ---- sums -> basis, each cell by one thread
             const float fine = __int_as_float((127 - (packed ? 16 - bits : 20 - shift)) << 23);
-            float2 F[2][kMBasis];
+            float2 F[Cfg::cells][kMBasis];
 #pragma unroll
-            for (int i = 0; i < 2; i++) {
+            for (int i = 0; i < Cfg::cells; i++) {
                 const int b = tid + i * kMThreads;
 #pragma unroll
                 for (int p = 0; p < kMBasis; p++) F[i][p] = make_float2(0.0f, 0.0f);
@@ -705,7 +718,7 @@ __global__ void __launch_bounds__(kMThreads, 2) ism_moment_kernel(const __grid_c
             }
             __syncthreads();   // sums read: the basis takes their place
 #pragma unroll
-            for (int i = 0; i < 2; i++) {
+            for (int i = 0; i < Cfg::cells; i++) {
                 const int b = tid + i * kMThreads;
                 if (b < nbe)
 #pragma unroll
@@ -724,7 +737,7 @@ __global__ void __launch_bounds__(kMThreads, 2) ism_moment_kernel(const __grid_c
                 float2 acc[16];
 #pragma unroll
                 for (int e = 0; e < 16; e++) acc[e] = make_float2(0.0f, 0.0f);
-                const unsigned char *cut = act == 1 ? P.cut1 : P.cut2;
+                const unsigned char *cut = P.cut[act == 1 ? 0 : 1];
                 int q = cut[g];
                 const int q_end = cut[g + 1];
                 int r = 0, base = 0;
@@ -767,7 +780,7 @@ __global__ void __launch_bounds__(kMThreads, 2) ism_moment_kernel(const __grid_c
         if (last && warp == 0) ctx_finish(s.ctx[par ^ 1], P, next, lane);
         __syncthreads();
         if (last && s.ctx[par ^ 1].valid)
-            axis_tables(P, s.ctx[par ^ 1], s.tab + (par ^ 1) * P.axis_cap, tid);
+            axis_tables<THREADS>(P, s.ctx[par ^ 1], s.tab + (par ^ 1) * P.axis_cap, tid);
         // ---- output: four samples per thread and round; round v of thread j takes the groups
         // t/4 = j + v kMThreads (mod kPowerThreads): the order in which the tail kernel sums the
         // window power
@@ -1130,8 +1143,9 @@ const MomBasis &moment_basis_cached(int tw) {
     if (it == known.end()) {
         it = known.emplace(tw, MomBasis{}).first;
         moment_basis(tw, it->second);
-        cut_filter(it->second, kMWarps, it->second.cut1);
-        cut_filter(it->second, kMWarps / 2, it->second.cut2);
+        for (int v = 0; v < 2; v++)
+            for (int tiles = 1; tiles <= 2; tiles++)
+                cut_filter(it->second, (v ? kMomSmall : kMomLarge) / 32 / tiles, it->second.cut[v][tiles - 1]);
     }
     return it->second;
 }
@@ -1139,34 +1153,43 @@ const MomBasis &moment_basis_cached(int tw) {
 // cells of a launch: the longest segment's outputs and the filter's reach past them
 int moment_cells(int T, const MomBasis &B) { return (T / 2 + 4 * B.quads + 8 + 7) / 8 * 8; }
 
-size_t moment_smem_bytes(int axis_cap, const MomBasis &B) {
+size_t moment_smem_bytes(int threads, int axis_cap, const MomBasis &B) {
     size_t o[9];
-    return mom_layout(B.n_quads, axis_cap, o);
+    return threads == kMomSmall ? mom_layout<MomCfg<kMomSmall>>(B.n_quads, axis_cap, o)
+                                : mom_layout<MomCfg<kMomLarge>>(B.n_quads, axis_cap, o);
 }
 
-int moment_blocks_per_sm(size_t smem) {
+static const void *moment_function(int threads) {
+    return threads == kMomSmall ? reinterpret_cast<const void *>(ism_moment_kernel<kMomSmall>)
+                                : reinterpret_cast<const void *>(ism_moment_kernel<kMomLarge>);
+}
+
+int moment_blocks_per_sm(int threads, size_t smem) {
     static std::mutex mu;
-    static std::map<size_t, int> known;
+    static std::map<std::pair<int, size_t>, int> known;
     std::lock_guard<std::mutex> lock(mu);
-    auto it = known.find(smem);
+    auto it = known.find({threads, smem});
     if (it != known.end()) return it->second;
     int n = 0;
-    cudaFuncSetAttribute(ism_moment_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, ism_moment_kernel, kMThreads, smem);
-    known[smem] = n;
+    cudaFuncSetAttribute(moment_function(threads), cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, moment_function(threads), threads, smem);
+    known[{threads, smem}] = n;
     return n;
 }
 
-cudaError_t moment_launch(const MomLaunch &p, size_t smem, int grid, cudaStream_t st) {
+cudaError_t moment_launch(const MomLaunch &p, int threads, size_t smem, int grid, cudaStream_t st) {
     static bool attr_set = false;   // per process; the attribute is per function
     if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(ism_moment_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        if (e != cudaSuccess) return e;
+        for (int t : {kMomSmall, kMomLarge}) {
+            cudaError_t e = cudaFuncSetAttribute(moment_function(t), cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+            if (e != cudaSuccess) return e;
+        }
         attr_set = true;
     }
     cudaError_t e = cudaMemsetAsync(p.work_counter, 0, sizeof(int), st);
     if (e != cudaSuccess) return e;
-    ism_moment_kernel<<<grid, kMThreads, smem, st>>>(p);
+    if (threads == kMomSmall) ism_moment_kernel<kMomSmall><<<grid, kMomSmall, smem, st>>>(p);
+    else ism_moment_kernel<kMomLarge><<<grid, kMomLarge, smem, st>>>(p);
     return cudaGetLastError();
 }
 

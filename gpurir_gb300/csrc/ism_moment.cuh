@@ -14,7 +14,9 @@ constexpr double kMomNear = 4.6;          // taps beyond this one pairs 0 to 2
 constexpr int kMomMinTw = 48;             // window lengths the moment path is used for
 constexpr int kMomMaxTw = 400;
 constexpr int kMomCells = 768;            // most cells of a segment
-constexpr int kMomWarps = 12;             // warps of a block
+constexpr int kMomLarge = 384, kMomSmall = 256;   // threads of a block: two per SM, three per SM
+constexpr int kMomSmallCells = 624;               // most cells of a segment with the latter
+constexpr int kMomTabSmem = 256;           // per-axis entries of a launch held in shared memory
 constexpr int kMomRuns = 18;               // three per pair
 
 // Quads (groups of four cell taps) of one basis pair.
@@ -29,7 +31,7 @@ struct MomBasis {
     float2 S[kMBasis][kMPairs];           // moments -> basis
     MomRun run[kMomRuns];
     int n_runs = 0, n_quads = 0;          // over all runs
-    unsigned char cut1[kMomWarps + 1], cut2[kMomWarps / 2 + 1];   // the warps' ranges of quads, for one tile or two
+    unsigned char cut[2][2][kMomLarge / 32 + 1];   // large, small blocks: the warps' ranges of quads, for one tile and two
     std::vector<float2> coef;             // 8 n_quads: per quad, tap by tap, two output phases
 };
 
@@ -48,7 +50,7 @@ struct MomLaunch {
     const float2 *coef;
     MomRun run[kMomRuns];
     int n_quads;
-    unsigned char cut1[kMomWarps + 1], cut2[kMomWarps / 2 + 1];
+    unsigned char cut[2][kMomLarge / 32 + 1];
     float2 S[kMBasis][kMPairs];
     // diffuse tail of the RIRs whose last segment is one item (TailArgs)
     uint64_t seed, offset;
@@ -61,8 +63,8 @@ struct MomLaunch {
 
 const MomBasis &moment_basis_cached(int tw);
 int moment_cells(int T, const MomBasis &B);
-size_t moment_smem_bytes(int axis_cap, const MomBasis &B);
-int moment_blocks_per_sm(size_t smem);
-cudaError_t moment_launch(const MomLaunch &p, size_t smem, int grid, cudaStream_t st);
+size_t moment_smem_bytes(int threads, int axis_cap, const MomBasis &B);
+int moment_blocks_per_sm(int threads, size_t smem);
+cudaError_t moment_launch(const MomLaunch &p, int threads, size_t smem, int grid, cudaStream_t st);
 
 }  // namespace gpurir

@@ -125,3 +125,23 @@ def test_absorbing_walls(built):
     room = [3.0, 4.0, 2.5]
     ps, pr, _ = _scene(11, room, 2, 2)
     _check(room, np.array([0.0, 0.0, 0.0, 0.0, 0.9, 0.8], np.float32), ps, pr, [9, 9, 15], 0.1, 16000.0)
+
+
+@pytest.mark.parametrize("fs,n_img", [(8000.0, 9), (16000.0, 9), (24000.0, 9), (16000.0, 64)])   # 24 kHz: the widest window
+@pytest.mark.parametrize("tail", [False, True])
+def test_launches_of_many_segments(built, fs, n_img, tail):
+    """Launches large enough for three blocks per SM, with the tail that their last items write;
+    64 images per axis: tables of nearly 200 entries."""
+    import gpurir_gb300 as G
+    room = [3.5, 3.0, 2.6]
+    ps, pr, beta = _scene(int(fs), room, 40, 36)
+    T, Td = 0.3 if tail else 0.2, 0.2
+    sim = G.Simulator(seed=5)
+    nb = [n_img, n_img, n_img + 1]
+    out = sim.simulate_rir(room, beta, ps, pr, None, None, 0, 0, nb, Td, T, fs)
+    for s, r in [(0, 0), (17, 20), (39, 35)]:
+        ref, parts = oracle.simulate_rir(room, beta, ps[s:s + 1], pr[r:r + 1], nb, T, fs, Td, seed=5, offset=0,
+                                         return_parts=True, rir_base=s * 36 + r)
+        n = parts["n_ism"]
+        assert rel_l2(out[s, r, :n], ref[0, 0, :n]) <= TOL
+        assert not tail or rel_l2(out[s, r, n:], ref[0, 0, n:]) <= 1e-4   # FP32 envelope and noise
