@@ -57,7 +57,7 @@ namespace gpurir {
 // The two shapes of a block: threads, blocks per SM, cells of one array (a constant, so that
 // offsets are immediates), groups of 32 images per batch of rows.  A block's phases (image
 // atomics, filter, output) wait for one another; three small blocks per SM overlap better
-// than two large ones.  128 rooms: 675 us with two, TIMES with three; 8 x 1024 array 370 and TIMES.  The
+// than two large ones.  128 rooms: 660 us with two, 617 with three; 64 x 32 array 370 and 327.  The
 // large one is for windows whose cells three blocks cannot hold and for launches of few
 // segments, where each item's fixed cost counts (plan_moment).
 template <int THREADS>
