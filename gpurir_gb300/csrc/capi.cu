@@ -685,7 +685,7 @@ static int plan_moment(gpurir_sim *s, const std::vector<RoomDesc> &R, Plan &P) {
     // Time of a launch whose segments are cut into parts of at most `limit` (cost of images), in
     // cost per slot: its heaviest item if one wave holds them all, else the mean load and, for
     // the uneven end, half a mean item; the launches that add parts up.
-    auto judge = [&](const Segs &segs, double slots, float rest, float limit, double &n) {
+    auto time_of = [&](const Segs &segs, double slots, float rest, float limit, double &n) {
         double total = 0.0;
         float worst = 0.0f, parts = 1.0f;
         n = 0.0;
@@ -723,7 +723,7 @@ static int plan_moment(gpurir_sim *s, const std::vector<RoomDesc> &R, Plan &P) {
                                          moment_blocks_per_sm(threads, moment_smem_bytes(threads, P.axis_cap, *P.mom)) < 3)) continue;
             auto consider = [&](float limit) {
                 double n;
-                const double t = blocks * judge(with, slots, rest, limit, n);
+                const double t = blocks * time_of(with, slots, rest, limit, n);
                 if (t < best) {
                     best = t;
                     part_limit = limit;
@@ -740,7 +740,7 @@ static int plan_moment(gpurir_sim *s, const std::vector<RoomDesc> &R, Plan &P) {
                 for (int it = 0; it < 12 && hi > 1.03 * lo; it++) {
                     const double mid = std::sqrt(lo * hi);
                     double items;
-                    judge(with, slots, rest, (float)mid, items);
+                    time_of(with, slots, rest, (float)mid, items);
                     (items <= slots ? hi : lo) = mid;
                 }
                 consider((float)hi);

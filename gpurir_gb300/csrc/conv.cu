@@ -1033,8 +1033,8 @@ __global__ void __launch_bounds__(M / 16) traj_adjoint_kernel(
 // spectral step stays in registers.  Work item = a run of block pairs of one point; the
 // run's part of dL/dx goes to `part` and a second kernel adds the runs in order.
 //
-// Forward and adjoint of the 400-point workload (3200 rows of 12800 samples) took 930 us with
-// whole rows and take 608 us with blocks, the adjoint alone ~565 and ~240; 500 MB of rows
+// The adjoint of the 400-point workload (3200 rows of 12800 samples) took 565 us with whole
+// rows and takes 199 us with blocks (at 73 % of the issue slots); 500 MB of rows
 // read and written are 75 us of that, the transforms' arithmetic the rest.
 constexpr int kBlk = 2048;                  // points of a block's transform
 constexpr int kBlkThreads = 128;

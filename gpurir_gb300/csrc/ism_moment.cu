@@ -32,15 +32,22 @@
 // change a bit: a moment is scaled by a power of two (from a bound on the segment's
 // amplitudes) to at most 2^20, rounded to an integer, and its remainder to 2^-20 of that to
 // a second one (both roundings by the addition of 1.5 2^23, whose bits are added up as they
-// are and removed by the count).  That is 41 bits below the segment's largest amplitude: more
-// than an FP32 sum keeps.  T_10 to T_13, whose taps' coefficients are below 5e-5, have the
-// first integer only.  An image too near for the bound (below 5 cm) goes into a short list and
-// is added in FP32 in a fixed order; a segment with more of those, or with cells of more
-// images than the integers hold, is done again with bounds that fit.
-// Shared-memory integer atomics take 2.7 cycles per warp at random cells (measured; an FP32
-// atomicAdd 9.3): 25 per image are what bounds a dense segment.  (Two other ways were built
-// first: a counting sort by cell with one thread per cell adding in image order needed 8
-// barriers per 1024 images and ran at 228 cycles per 32 images and SM.)
+// are and removed by the count): 41 bits below the segment's largest amplitude.  T_8 to
+// T_13, whose taps' coefficients are below 2e-3, have the first integer only.  Cells of up to
+// 448 images need fewer guard bits and share words (kMPSums below): 17 words a cell instead
+// of 23, 28 to 31 bits below the bound, which follows the attenuation of each segment.  An
+// image too near for the bound (below 5 cm) goes into a short list and is added in FP32 in
+// a fixed order; a segment with more of those, or with cells of more images than the
+// integers hold, is done again with bounds that fit.
+//
+// What bounds it: the shared-memory atomics of the image loop (2.7 cycles per warp at random
+// cells, 3.6 wavefronts; an FP32 atomicAdd takes 9.3 cycles) where images are many -- the
+// load pipe is at 77 % on 128 rooms -- and issue with the phases' barriers where they are few
+// (56 % of the slots on the array).  Per launch, ism_forward.cu and this kernel: one dense RIR of
+// 6 million images 531 and 98 us, 64 x 32 array 490 and 327, 128 rooms 2620 and 617, 15 RIRs at
+// 48 kHz 87 and 40.  (Other ways that were built first: a counting sort by cell with one
+// thread per cell adding in image order needed 8 barriers per 1024 images and ran at 228
+// cycles per 32 images and SM, against 90 here.)
 #include <algorithm>
 #include <cmath>
 #include <cstddef>
