@@ -466,6 +466,9 @@ __global__ void __launch_bounds__(THREADS, MomCfg<THREADS>::blocks) ism_moment_k
                 my_rows = n_box > C.it.i_lo ? (n_box - C.it.i_lo + C.it.i_hi - 1) / C.it.i_hi : 0;
             }
             const float rW1 = 1.0f / (float)max(W1, 1);
+            // (in registers: the atomics might alias the context, so that it would be read again per image)
+            const int kind = R.spkr | R.mic << 8 | (R.ref_delay != 0) << 16;
+            const ff k_samples = {R.kh, R.kl};
             const int batch = min(Cfg::rows, 32 * Cfg::groups / N2);   // rows at once: their images fill the groups at most
             // mean images per cell at the segment's end: a room's volume holds one; cells with few
             // have packed sums
@@ -566,8 +569,8 @@ __global__ void __launch_bounds__(THREADS, MomCfg<THREADS>::blocks) ism_moment_k
                         ff d2 = ff_add(ff{row.x, row.y}, ff{t2.x, t2.y});
                         float v0h = 0.0f, v1h = 0.0f;
                         const int m0 = __float_as_int(row.w) & 0xffff, m1 = __float_as_int(row.w) >> 16;
-                        const int spkr = R.spkr, mic = R.mic;
-                        const bool ref_delay = R.ref_delay != 0, ref_dir = spkr != P_OMNI || mic != P_OMNI;
+                        const int spkr = kind & 255, mic = kind >> 8 & 255;
+                        const bool ref_delay = kind >> 16 != 0, ref_dir = (kind & 0xffff) != (P_OMNI | P_OMNI << 8);
                         if (ref_dir || ref_delay) {
                             v0h = tab[m0].z;
                             v1h = tab[N0 + m1].z;
@@ -576,7 +579,7 @@ __global__ void __launch_bounds__(THREADS, MomCfg<THREADS>::blocks) ism_moment_k
                         const float rs0 = rsqrt_approx(d2.hi);
                         float inv_d;
                         const ff dist = ff_dist_newton(d2, rs0, d2.hi * rs0, inv_d);
-                        const ff tau = ref_delay ? ff{ref_tau(d2.hi, R.c, R.fs), 0.0f} : ff_mul(dist, ff{R.kh, R.kl});
+                        const ff tau = ref_delay ? ff{ref_tau(d2.hi, R.c, R.fs), 0.0f} : ff_mul(dist, k_samples);
                         float amp = row.z * t2.w * (0.0795774715459476679f * inv_d);   // attenuation / (4 pi dist)
                         if (spkr != P_OMNI) {
                             // doa = image -> receiver, axis mirrored per reflection (:357-362)
