@@ -73,14 +73,14 @@ int traj_adjoint_blk_fft();
 cudaError_t traj_adjoint_blk_launch(const double *g, long n_out, const int *w_ini, const int *w_len, const float *seg,
                                     const float *rir, int P, int R, int L, int S, const BlkPlan &b, const float2 *W,
                                     float *gt, float *work, float *grad_rir, float *grad_sig, cudaStream_t st);
-cudaError_t room_beta_launch(RoomDesc *rooms, int n_rooms, const float *beta, cudaStream_t st);
+cudaError_t room_beta_launch(RoomDesc *rooms, int n_rooms, const float *beta, int *ctl, cudaStream_t st);
 int l2_grad_blocks(long n);
 int tuning(int knob);
 cudaError_t l2_grad_launch(const float *y, const float *t, long n, float scale, float *g, double *partial,
-                           float *loss, cudaStream_t st);
+                           float *loss, int *done, cudaStream_t st);
 cudaError_t room_beta_skip_launch(RoomDesc *rooms, int n_rooms, const float *beta, const IsmItem *items,
                                   int n_items, const float *pos_src, const float *pos_rcv, unsigned char *skip,
-                                  cudaStream_t st);
+                                  int *ctl, cudaStream_t st);
 }  // namespace gpurir
 
 using namespace gpurir;
@@ -135,7 +135,7 @@ struct gpurir_sim {
     bool stage_pending = false;
     cudaEvent_t ws_busy = nullptr;   // recorded after the last use of d_ws
     bool ws_recorded = false;
-    int *d_ctl = nullptr;      // [0] work counter, [1] status
+    int *d_ctl = nullptr;      // [0] work counter (one-shot adjoint), [1] status
     int *h_ctl = nullptr;      // pinned copy of the status word
     long last_n_rir = 0;
     size_t env_off = 0;        // offset of the envelope array in d_ws
@@ -863,7 +863,7 @@ static int check_status(gpurir_sim *s) {
 
 // Byte layout of one launch's descriptors (mirrored host staging -> device).
 struct Layout {
-    size_t o_rooms, o_items, o_rirs, o_groups, o_coef, o_pos, o_pre, stage_bytes, o_env, o_axis, o_part, o_skip, o_out,
+    size_t o_rooms, o_work, o_items, o_rirs, o_groups, o_coef, o_pos, o_pre, stage_bytes, o_env, o_axis, o_part, o_skip, o_out,
         dev_bytes;
 };
 
@@ -872,7 +872,9 @@ static Layout make_layout(const Plan &P, size_t n_rooms, long n_src, long n_rcv,
     Layout L;
     // rooms and positions first: the part of an upload that changes from call to call
     L.o_rooms = 0;
-    L.o_pos = align_up(L.o_rooms + n_rooms * sizeof(RoomDesc), 256);
+    // work counter, zero in every upload: no memset per call (a plain room 82 to 74 us)
+    L.o_work = align_up(n_rooms * sizeof(RoomDesc), 16);
+    L.o_pos = align_up(L.o_work + 16, 256);
     size_t n_pos = host_io ? (size_t)(n_src + n_rcv) * 3 * 2 : 0;
     L.o_pre = align_up(L.o_pos + n_pos * sizeof(float), 256);   // per-RIR silent-tail flags (host I/O)
     L.o_items = align_up(L.o_pre + (host_io ? (size_t)M : 0), 256);
@@ -928,8 +930,12 @@ static std::vector<double> plan_key(const gpurir_sim *s, const std::vector<RoomD
     return k;
 }
 
-static void fill_stage(char *h, const Layout &L, const std::vector<RoomDesc> &R, const Plan &P) {
+static void fill_rooms(char *h, const Layout &L, const std::vector<RoomDesc> &R) {
     memcpy(h + L.o_rooms, R.data(), R.size() * sizeof(RoomDesc));
+    memset(h + L.o_work, 0, 16);
+}
+static void fill_stage(char *h, const Layout &L, const std::vector<RoomDesc> &R, const Plan &P) {
+    fill_rooms(h, L, R);
     if (!P.items.empty()) memcpy(h + L.o_items, P.items.data(), P.items.size() * sizeof(IsmItem));
     if (!P.rirs.empty()) memcpy(h + L.o_rirs, P.rirs.data(), P.rirs.size() * sizeof(IsmItem));
     if (!P.groups.empty()) memcpy(h + L.o_groups, P.groups.data(), P.groups.size() * sizeof(PartGroup));
@@ -1164,7 +1170,7 @@ static int simulate_rooms(gpurir_sim *s, std::vector<RoomDesc> &R, long n_src, l
     const bool items_resident = hit && s->pcache->gen == s->ws_gen;
     const size_t up_bytes = items_resident ? L.o_items : L.stage_bytes;
     char *h = s->h_stage;
-    if (items_resident) memcpy(h + L.o_rooms, R.data(), R.size() * sizeof(RoomDesc));
+    if (items_resident) fill_rooms(h, L, R);
     else fill_stage(h, L, R, P);
     const float *dps = pos_src, *dpr = pos_rcv, *dos = orV_src, *dor = orV_rcv;
     char *d = s->d_ws;
@@ -1200,13 +1206,13 @@ static int simulate_rooms(gpurir_sim *s, std::vector<RoomDesc> &R, long n_src, l
     CK(cudaEventRecord(s->stage_done, st));
     s->stage_pending = true;
     if (!items_resident) s->pcache->gen = ++s->ws_gen;
-    if (d_beta) CK(room_beta_launch(reinterpret_cast<RoomDesc *>(d + L.o_rooms), (int)R.size(), d_beta, st));
+    if (d_beta) CK(room_beta_launch(reinterpret_cast<RoomDesc *>(d + L.o_rooms), (int)R.size(), d_beta, nullptr, st));
     float *dout = host_io ? (direct ? hout : reinterpret_cast<float *>(d + L.o_out)) : out;
     s->last_direct = direct;
     s->ev_ism = s->ev_tail = false;
     s->last_h2d = up_bytes;
     s->last_d2h = sizeof(int) + (host_io ? (uint64_t)out_elems * sizeof(float) : 0);
-    if ((rc = enqueue_kernels(s, P, d, L, M, dps, dpr, dos, dor, dout, s->d_ctl, nullptr, st, true, false,
+    if ((rc = enqueue_kernels(s, P, d, L, M, dps, dpr, dos, dor, dout, reinterpret_cast<int *>(d + L.o_work), nullptr, st, true, false,
                               pre ? reinterpret_cast<const unsigned char *>(d + L.o_pre) : nullptr)))
         return rc;
     if (pre) CK(cudaStreamWaitEvent(st, s->side_done, 0));   // the call ends after the streamed tails
@@ -1466,6 +1472,7 @@ extern "C" int gpurir_batch_create(gpurir_sim *s, int n_rooms, const gpurir_room
     uint64_t *offset = reinterpret_cast<uint64_t *>(b->d + o_ctl + 8);
     e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
+        cudaMemsetAsync(counter, 0, sizeof(int), cap);   // (a failure shows at the end of the capture)
         rc = enqueue_kernels(s, P, b->d, L, M, d_pos_src, d_pos_rcv, d_orV_src, d_orV_rcv, d_out,
                              counter, offset, cap, false);
         if (rc == GPURIR_OK && P.max_n_diff > 0) {
@@ -1664,12 +1671,13 @@ static int backward_batch(gpurir_sim *s, int n_rooms, const gpurir_room *rooms, 
     s->ws_gen++;   // the cached plan's items were overwritten
     CK(cudaEventRecord(s->stage_done, st));
     s->stage_pending = true;
-    if (d_beta) CK(room_beta_launch(reinterpret_cast<RoomDesc *>(d + o_rooms), n_rooms, d_beta, st));
+    if (d_beta) CK(room_beta_launch(reinterpret_cast<RoomDesc *>(d + o_rooms), n_rooms, d_beta, nullptr, st));
     float *ig = reinterpret_cast<float *>(d + o_ig);
     if (n_items == 0) {
         CK(cudaMemsetAsync(ig, 0, 18 * sizeof(float), st));
     } else {
         const int grid = std::min(n_items, s->num_sms * bps);
+        CK(cudaMemsetAsync(s->d_ctl, 0, sizeof(int), st));
         CK(ism_backward_launch(P.tpl, reinterpret_cast<const RoomDesc *>(d + o_rooms),
                                reinterpret_cast<const IsmItem *>(d + o_items), n_items, d_pos_src,
                                d_pos_rcv, d_orV_src, d_orV_rcv, d_grad_rir, ig, s->d_ctl, s->d_ctl + 1,
@@ -1768,7 +1776,7 @@ extern "C" int gpurir_adjoint_create(gpurir_sim *s, int n_rooms, const gpurir_ro
     a->o_ig = off;
     a->o_bitems = align_up(a->o_ig + (size_t)std::max(n_items, 1) * 18 * sizeof(float), 256);
     a->o_ctl = align_up(a->o_bitems + bitems.size() * sizeof(IsmItem), 256);
-    const size_t bytes = a->o_ctl + 256;   // [0] forward counter, [1] adjoint counter, [2] status, +16 call offset
+    const size_t bytes = a->o_ctl + 256;   // [0] forward counter, [1] adjoint counter, [2] status, [3] loss blocks, +16 call offset
     std::vector<char> h(a->o_ctl + 256, 0);
     fill_stage(h.data(), a->L, R, P);
     for (int k = 0; k < 6; k++)
@@ -1799,9 +1807,9 @@ extern "C" int gpurir_adjoint_forward(gpurir_adjoint *a, const float *d_beta, co
     if (fuse_skip)   // room tables and the items' skip flags in one launch
         CK(room_beta_skip_launch(reinterpret_cast<RoomDesc *>(a->d + a->L.o_rooms), a->n_rooms, d_beta,
                                  reinterpret_cast<const IsmItem *>(a->d + a->L.o_items), (int)a->P.items.size(),
-                                 d_pos_src, d_pos_rcv, reinterpret_cast<unsigned char *>(a->d + a->L.o_skip), st));
+                                 d_pos_src, d_pos_rcv, reinterpret_cast<unsigned char *>(a->d + a->L.o_skip), ctl, st));
     else
-        CK(room_beta_launch(reinterpret_cast<RoomDesc *>(a->d + a->L.o_rooms), a->n_rooms, d_beta, st));
+        CK(room_beta_launch(reinterpret_cast<RoomDesc *>(a->d + a->L.o_rooms), a->n_rooms, d_beta, ctl, st));
     a->rooms_written = true;
     int rc = enqueue_kernels(a->sim, a->P, a->d, a->L, a->M, d_pos_src, d_pos_rcv, d_orV_src, d_orV_rcv,
                              d_out, ctl, offset, st, false, fuse_skip);
@@ -1810,11 +1818,11 @@ extern "C" int gpurir_adjoint_forward(gpurir_adjoint *a, const float *d_beta, co
     return GPURIR_OK;
 }
 
-extern "C" int gpurir_adjoint_backward(gpurir_adjoint *a, const float *d_beta, const float *d_pos_src,
-                                       const float *d_pos_rcv, const float *d_orV_src,
-                                       const float *d_orV_rcv, const float *d_grad_rir, float *d_grad_beta,
-                                       float *d_grad_pos_src, float *d_grad_pos_rcv, float *d_grad_orV_src,
-                                       float *d_grad_orV_rcv, void *stream) {
+// ready: the work counter is 0 (a forward has just been enqueued before)
+static int adjoint_backward(gpurir_adjoint *a, const float *d_beta, const float *d_pos_src, const float *d_pos_rcv,
+                            const float *d_orV_src, const float *d_orV_rcv, const float *d_grad_rir,
+                            float *d_grad_beta, float *d_grad_pos_src, float *d_grad_pos_rcv,
+                            float *d_grad_orV_src, float *d_grad_orV_rcv, void *stream, bool ready) {
     if (!a || !d_pos_src || !d_pos_rcv || !d_grad_rir) return fail(GPURIR_ERR_INVALID, "NULL argument");
     if (!d_beta && !a->rooms_written)
         return fail(GPURIR_ERR_INVALID, "d_beta is NULL but no forward call has written the room tables");
@@ -1826,7 +1834,8 @@ extern "C" int gpurir_adjoint_backward(gpurir_adjoint *a, const float *d_beta, c
     const int n_items = a->n_bitems;
     float *ig = reinterpret_cast<float *>(a->d + a->o_ig);
     const RoomDesc *drooms = reinterpret_cast<const RoomDesc *>(a->d + a->L.o_rooms);
-    if (d_beta) CK(room_beta_launch(reinterpret_cast<RoomDesc *>(a->d + a->L.o_rooms), a->n_rooms, d_beta, st));
+    if (d_beta) CK(room_beta_launch(reinterpret_cast<RoomDesc *>(a->d + a->L.o_rooms), a->n_rooms, d_beta, ctl, st));
+    else if (!ready) CK(cudaMemsetAsync(ctl + 1, 0, sizeof(int), st));
     if (n_items == 0) {
         CK(cudaMemsetAsync(ig, 0, 18 * sizeof(float), st));
     } else {
@@ -1839,6 +1848,15 @@ extern "C" int gpurir_adjoint_backward(gpurir_adjoint *a, const float *d_beta, c
     float *const outs[5] = {d_grad_beta, d_grad_pos_src, d_grad_pos_rcv, d_grad_orV_src, d_grad_orV_rcv};
     CK(grad_reduce_launch(ig, dp, a->n_rooms, (int)a->ns, (int)a->nr, outs, st));
     return GPURIR_OK;
+}
+
+extern "C" int gpurir_adjoint_backward(gpurir_adjoint *a, const float *d_beta, const float *d_pos_src,
+                                       const float *d_pos_rcv, const float *d_orV_src,
+                                       const float *d_orV_rcv, const float *d_grad_rir, float *d_grad_beta,
+                                       float *d_grad_pos_src, float *d_grad_pos_rcv, float *d_grad_orV_src,
+                                       float *d_grad_orV_rcv, void *stream) {
+    return adjoint_backward(a, d_beta, d_pos_src, d_pos_rcv, d_orV_src, d_orV_rcv, d_grad_rir, d_grad_beta,
+                            d_grad_pos_src, d_grad_pos_rcv, d_grad_orV_src, d_grad_orV_rcv, stream, false);
 }
 
 extern "C" int gpurir_adjoint_l2_step(gpurir_adjoint *a, const float *d_beta, const float *d_pos_src,
@@ -1856,10 +1874,11 @@ extern "C" int gpurir_adjoint_l2_step(gpurir_adjoint *a, const float *d_beta, co
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     int rc = gpurir_adjoint_forward(a, d_beta, d_pos_src, d_pos_rcv, d_orV_src, d_orV_rcv, d_out, stream);
     if (rc) return rc;
-    CK(l2_grad_launch(d_out, d_target, (long)a->out_elems, scale, a->d_g, a->d_partial, d_loss, st));
+    CK(l2_grad_launch(d_out, d_target, (long)a->out_elems, scale, a->d_g, a->d_partial, d_loss,
+                      reinterpret_cast<int *>(a->d + a->o_ctl) + 3, st));
     // the room tables of the forward just enqueued serve the adjoint (same beta)
-    return gpurir_adjoint_backward(a, nullptr, d_pos_src, d_pos_rcv, d_orV_src, d_orV_rcv, a->d_g, d_grad_beta,
-                                   d_grad_pos_src, d_grad_pos_rcv, d_grad_orV_src, d_grad_orV_rcv, stream);
+    return adjoint_backward(a, nullptr, d_pos_src, d_pos_rcv, d_orV_src, d_orV_rcv, a->d_g, d_grad_beta,
+                            d_grad_pos_src, d_grad_pos_rcv, d_grad_orV_src, d_grad_orV_rcv, stream, true);
 }
 
 extern "C" int gpurir_adjoint_status(gpurir_adjoint *a, int *status) {

@@ -509,8 +509,6 @@ cudaError_t ism_backward_launch(int tpl, const RoomDesc *rooms, const IsmItem *i
     p.max_tseg = max_tseg;
     p.pad = 64 * tpl;   // >= 2 * 32 * TPL reach of the taps on either side
     size_t smem = ism_backward_smem_bytes(tpl, max_tseg, p.pad, axis_cap);
-    cudaError_t e = cudaMemsetAsync(work_counter, 0, sizeof(int), st);
-    if (e != cudaSuccess) return e;
     // taps beyond |x| < Tw/2 exist only when the window does not fill the lanes exactly
     switch (tpl * 2 + (clamp ? 1 : 0)) {
     case 4: return bwd_tpl<2, false>(p, grid, smem, st);

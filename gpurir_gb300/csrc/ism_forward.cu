@@ -51,7 +51,7 @@ struct IsmLaunch {
     const float *pos_src, *pos_rcv;   // [*, 3]
     const float *orv_src, *orv_rcv;   // [*, 3] (unused for omni rooms)
     float *out;
-    int *work_counter;                // reset to 0 before every launch
+    int *work_counter;                // 0 at every launch (the caller's upload or the kernel before)
     int *status;                      // device error word
     int em;                           // pad words before/after the buffers
     int max_nsub;                     // sub-ranges this launch's smem holds
@@ -890,8 +890,6 @@ cudaError_t ism_forward_launch(int tpl, const RoomDesc *rooms, const IsmItem *it
     p.out = out; p.work_counter = work_counter; p.status = status;
     p.em = em; p.max_nsub = max_nsub; p.clamp = clamp; p.tw = tw;
     size_t smem = ism_forward_smem_bytes(tpl, em, max_nsub, mode, tw);
-    cudaError_t e = cudaMemsetAsync(work_counter, 0, sizeof(int), st);
-    if (e != cudaSuccess) return e;
     switch (mode) {
     case kModeF32: return launch_mode<kModeF32>(tpl, p, grid, smem, st);
     case kModeMP: return launch_mode<kModeMP>(tpl, p, grid, smem, st);

@@ -1196,8 +1196,6 @@ cudaError_t moment_launch(const MomLaunch &p, int threads, size_t smem, int grid
         }
         attr_set = true;
     }
-    cudaError_t e = cudaMemsetAsync(p.work_counter, 0, sizeof(int), st);
-    if (e != cudaSuccess) return e;
     if (threads == kMomSmall) ism_moment_kernel<kMomSmall><<<grid, kMomSmall, smem, st>>>(p);
     else ism_moment_kernel<kMomLarge><<<grid, kMomLarge, smem, st>>>(p);
     return cudaGetLastError();

@@ -3,8 +3,8 @@
 // For a training loop that fits RIRs to a target (the inverse problem: walls
 // and positions from measured responses), loss = scale * sum (y - t)^2 and
 // dL/dy = 2 scale (y - t) are formed by one kernel that reads y and t once
-// and writes the gradient the adjoint kernel consumes; a second one-block
-// kernel adds the per-block partial sums in a fixed order (deterministic).
+// and writes the gradient the adjoint kernel consumes; its last block to finish
+// adds the per-block partial sums in a fixed order (deterministic).
 // gpuRIR has no counterpart (it is not differentiable).
 #include <cuda_runtime.h>
 
@@ -24,12 +24,15 @@ __device__ __forceinline__ double block_sum(double v, double *red) {
     return s;   // valid in thread 0
 }
 
-// g = 2 scale (y - t); partial[block] = sum over the block's elements of (y - t)^2.
+// g = 2 scale (y - t); partial[block] = sum over the block's elements of (y - t)^2; *loss = scale
+// times their sum, by the block that finishes last (*done counts them from 0; a launch of
+// its own for this sum stood between the gradient and the adjoint).
 __global__ void __launch_bounds__(kLossThreads) l2_grad_kernel(const float *__restrict__ y,
                                                                const float *__restrict__ t, long n,
                                                                float scale, float *__restrict__ g,
-                                                               double *__restrict__ partial) {
+                                                               double *partial, float *__restrict__ loss, int *done) {
     __shared__ double red[kLossThreads / 32];
+    __shared__ int last;
     const float two_s = 2.0f * scale;
     float acc = 0.0f;
     const long stride = (long)gridDim.x * kLossThreads;
@@ -50,16 +53,18 @@ __global__ void __launch_bounds__(kLossThreads) l2_grad_kernel(const float *__re
             g[i] = two_s * d;
         }
     const double s = block_sum((double)acc, red);
-    if (threadIdx.x == 0) partial[blockIdx.x] = s;
-}
-
-__global__ void __launch_bounds__(kLossThreads) l2_final_kernel(const double *__restrict__ partial, int n_part,
-                                                                float scale, float *__restrict__ loss) {
-    __shared__ double red[kLossThreads / 32];
+    if (threadIdx.x == 0) {
+        partial[blockIdx.x] = s;
+        __threadfence();
+        last = atomicAdd(done, 1) == (int)gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
     double v = 0.0;
-    for (int i = threadIdx.x; i < n_part; i += kLossThreads) v += partial[i];
-    const double s = block_sum(v, red);
-    if (threadIdx.x == 0) *loss = (float)(s * (double)scale);
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += kLossThreads) v += __ldcg(&partial[i]);
+    const double sum = block_sum(v, red);
+    if (threadIdx.x == 0) *loss = (float)(sum * (double)scale);
 }
 
 // Blocks of l2_grad_kernel for n elements (fixed for a given n: the sum order, and so
@@ -71,15 +76,12 @@ int l2_grad_blocks(long n) {
     return (int)b;
 }
 
-// y, t, g must be 16-byte aligned; partial holds l2_grad_blocks(n) doubles.
+// y, t, g must be 16-byte aligned; partial holds l2_grad_blocks(n) doubles, *done is 0.
 cudaError_t l2_grad_launch(const float *y, const float *t, long n, float scale, float *g, double *partial,
-                           float *loss, cudaStream_t st) {
+                           float *loss, int *done, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
     const int blocks = l2_grad_blocks(n);
-    l2_grad_kernel<<<blocks, kLossThreads, 0, st>>>(y, t, n, scale, g, partial);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    l2_final_kernel<<<1, kLossThreads, 0, st>>>(partial, blocks, scale, loss);
+    l2_grad_kernel<<<blocks, kLossThreads, 0, st>>>(y, t, n, scale, g, partial, loss, done);
     return cudaGetLastError();
 }
 
