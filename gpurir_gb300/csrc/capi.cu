@@ -135,8 +135,10 @@ struct gpurir_sim {
     bool stage_pending = false;
     cudaEvent_t ws_busy = nullptr;   // recorded after the last use of d_ws
     bool ws_recorded = false;
-    int *d_ctl = nullptr;      // [0] work counter (one-shot adjoint), [1] status
-    int *h_ctl = nullptr;      // pinned copy of the status word
+    int *d_ctl = nullptr;      // [0] work counter, [1] status, of the one-shot adjoint
+    // [1] status of the image-source kernels, page-locked: a kernel that rejects an item stores there,
+    // and no call copies a status word back (a plain room 74 to 68 us)
+    int *h_ctl = nullptr;
     long last_n_rir = 0;
     size_t env_off = 0;        // offset of the envelope array in d_ws
     int profile = 0;           // record events around each kernel
@@ -194,6 +196,7 @@ extern "C" int gpurir_create(int mixed_precision, int lookup_table, uint64_t see
     if (e == cudaSuccess) e = cudaMalloc(&s->d_ctl, 4 * sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(s->d_ctl, 0, 4 * sizeof(int));
     if (e == cudaSuccess) e = cudaMallocHost(&s->h_ctl, 4 * sizeof(int));
+    if (e == cudaSuccess) memset(s->h_ctl, 0, 4 * sizeof(int));
     if (e != cudaSuccess) {
         std::string msg = std::string("gpurir_create: ") + cudaGetErrorString(e);
         gpurir_destroy(s);
@@ -853,9 +856,9 @@ static int plan_rooms(gpurir_sim *s, const std::vector<RoomDesc> &R, Plan &P) {
 }
 
 static int check_status(gpurir_sim *s) {
-    if (s->h_ctl[1] != 0) {
-        int code = s->h_ctl[1];
-        cudaMemsetAsync(s->d_ctl + 1, 0, sizeof(int), s->stream);
+    const int code = *(volatile int *)(s->h_ctl + 1);
+    if (code != 0) {
+        s->h_ctl[1] = 0;
         return fail(GPURIR_ERR_DEVICE, "kernel rejected a work item (code " + std::to_string(code) + ")");
     }
     return GPURIR_OK;
@@ -977,7 +980,7 @@ static int enqueue_kernels(gpurir_sim *s, const Plan &P, const char *d, const La
         m.out = dout;
         m.partial = reinterpret_cast<float *>(const_cast<char *>(d) + L.o_part);
         m.work_counter = work_counter;
-        m.status = s->d_ctl + 1;
+        m.status = s->h_ctl + 1;
         m.axis_tab = reinterpret_cast<float4 *>(const_cast<char *>(d) + L.o_axis);
         m.axis_cap = P.axis_cap;
         m.T = P.mom_T;
@@ -996,7 +999,7 @@ static int enqueue_kernels(gpurir_sim *s, const Plan &P, const char *d, const La
     } else if (P.grid > 0)
         CK(ism_forward_launch(P.tpl, drooms, reinterpret_cast<const IsmItem *>(d + L.o_items),
                               (int)P.items.size(), dps, dpr, dos, dor, dout, work_counter,
-                              s->d_ctl + 1, P.em, P.nsub, P.clamp, P.grid, st, P.mode, P.tw, &ta,
+                              s->h_ctl + 1, P.em, P.nsub, P.clamp, P.grid, st, P.mode, P.tw, &ta,
                               reinterpret_cast<float4 *>(const_cast<char *>(d) + L.o_axis), P.axis_cap,
                               reinterpret_cast<float *>(const_cast<char *>(d) + L.o_part), skip));
     if (!P.groups.empty()) {   // RIRs split by images: add up their partial segments
@@ -1211,7 +1214,7 @@ static int simulate_rooms(gpurir_sim *s, std::vector<RoomDesc> &R, long n_src, l
     s->last_direct = direct;
     s->ev_ism = s->ev_tail = false;
     s->last_h2d = up_bytes;
-    s->last_d2h = sizeof(int) + (host_io ? (uint64_t)out_elems * sizeof(float) : 0);
+    s->last_d2h = host_io ? (uint64_t)out_elems * sizeof(float) : 0;
     if ((rc = enqueue_kernels(s, P, d, L, M, dps, dpr, dos, dor, dout, reinterpret_cast<int *>(d + L.o_work), nullptr, st, true, false,
                               pre ? reinterpret_cast<const unsigned char *>(d + L.o_pre) : nullptr)))
         return rc;
@@ -1219,7 +1222,6 @@ static int simulate_rooms(gpurir_sim *s, std::vector<RoomDesc> &R, long n_src, l
     s->env_off = L.o_env;
     s->last_n_rir = P.max_n_diff > 0 ? M : 0;
     s->calls++;
-    CK(cudaMemcpyAsync(s->h_ctl + 1, s->d_ctl + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
     if (host_io && !direct)
         CK(cudaMemcpyAsync(out, dout, (size_t)out_elems * sizeof(float), cudaMemcpyDeviceToHost, st));
     CK(cudaEventRecord(s->ws_busy, st));
@@ -1525,9 +1527,11 @@ extern "C" int gpurir_batch_destroy(gpurir_batch *b) {
 extern "C" int gpurir_device_status(gpurir_sim *s) {
     if (!s) return fail(GPURIR_ERR_INVALID, "NULL handle");
     int v = 0;
-    CK(cudaMemcpy(&v, s->d_ctl + 1, sizeof(int), cudaMemcpyDeviceToHost));
+    CK(cudaMemcpy(&v, s->d_ctl + 1, sizeof(int), cudaMemcpyDeviceToHost));   // (the one-shot adjoint's)
+    if (v == 0) v = *(volatile int *)(s->h_ctl + 1);
     if (v != 0) {
         CK(cudaMemset(s->d_ctl + 1, 0, sizeof(int)));
+        s->h_ctl[1] = 0;
         return fail(GPURIR_ERR_DEVICE, "kernel rejected a work item (code " + std::to_string(v) + ")");
     }
     return GPURIR_OK;
