@@ -8,6 +8,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "launch.cuh"
+
 namespace gpurir {
 
 // Polar patterns, numbering of src/gpuRIR_cuda.h:2-8.

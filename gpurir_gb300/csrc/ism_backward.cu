@@ -68,6 +68,7 @@ __device__ __forceinline__ float pattern_slope(int pattern) {
 
 template <int TPL, bool CLAMP>
 __global__ void __launch_bounds__(kBThreads, 3) ism_backward_kernel(BwdLaunch P) {
+    after_previous();
     // per-warp scratch of 32 kept images: records, then A and B of each
     extern __shared__ __align__(16) unsigned char smem_raw[];
     // records of the kept images: (sigma, f, cos phi, sin phi) and
@@ -448,6 +449,7 @@ struct GradSets {
 constexpr int kRedThreads = 128;
 
 __global__ void __launch_bounds__(kRedThreads) grad_reduce_kernel(const float *item_grad, GradSets G) {
+    after_previous();
     __shared__ float red[kRedThreads / 32][6];
     int t = blockIdx.x, k = 0;
     while (k < 5 && t >= G.s[k].n_target) t -= G.s[k++].n_target;
@@ -492,8 +494,7 @@ static cudaError_t bwd_tpl(const BwdLaunch &p, int grid, size_t smem, cudaStream
         if (e != cudaSuccess) return e;
         attr_set = true;
     }
-    ism_backward_kernel<TPL, CLAMP><<<grid, kBThreads, smem, st>>>(p);
-    return cudaGetLastError();
+    return launch_after(ism_backward_kernel<TPL, CLAMP>, grid, kBThreads, smem, st, p);
 }
 
 cudaError_t ism_backward_launch(int tpl, const RoomDesc *rooms, const IsmItem *items, int n_items,
@@ -542,8 +543,7 @@ cudaError_t grad_reduce_launch(const float *item_grad, const int *const csr[6], 
     }
     if (targets <= 0) return cudaSuccess;
     if (targets > 0x7fffffffL) return cudaErrorInvalidValue;
-    grad_reduce_kernel<<<(unsigned)targets, kRedThreads, 0, st>>>(item_grad, G);
-    return cudaGetLastError();
+    return launch_after(grad_reduce_kernel, (unsigned)targets, kRedThreads, 0, st, item_grad, G);
 }
 
 // Resident blocks per SM of the adjoint kernel with `smem` bytes of shared memory.

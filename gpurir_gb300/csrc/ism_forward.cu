@@ -209,6 +209,7 @@ __device__ __forceinline__ void scatter_list(float *bs, int origin, const float4
 
 template <int TPL, int MODE_ARG>
 __global__ void __launch_bounds__(kThreads, 2) ism_forward_kernel(IsmLaunch P) {
+    after_previous();
     constexpr int MODE = MODE_ARG & 3;                  // tap evaluation
     constexpr bool COMP = (MODE_ARG & kModeComp) != 0;  // compensated accumulation across chunks
     constexpr int KS = 32 * TPL;   // taps per image, rounded up to the warp
@@ -811,8 +812,7 @@ static cudaError_t launch_tpl(const IsmLaunch &p, int grid, size_t smem, cudaStr
         if (e != cudaSuccess) return e;
         attr_set = true;
     }
-    ism_forward_kernel<TPL, MODE><<<grid, kThreads, smem, st>>>(p);
-    return cudaGetLastError();
+    return launch_after(ism_forward_kernel<TPL, MODE>, grid, kThreads, smem, st, p);
 }
 
 template <int MODE>
@@ -905,6 +905,7 @@ cudaError_t ism_forward_launch(int tpl, const RoomDesc *rooms, const IsmItem *it
 // First segments are not tested (they hold the direct path).
 __global__ void item_skip_kernel(const RoomDesc *rooms, const IsmItem *items, int n_items, const float *pos_src,
                                  const float *pos_rcv, unsigned char *skip) {
+    after_previous();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n_items) return;
     const IsmItem it = items[k];
@@ -921,13 +922,13 @@ __global__ void item_skip_kernel(const RoomDesc *rooms, const IsmItem *items, in
 cudaError_t item_skip_launch(const RoomDesc *rooms, const IsmItem *items, int n_items, const float *pos_src,
                              const float *pos_rcv, unsigned char *skip, cudaStream_t st) {
     if (n_items <= 0) return cudaSuccess;
-    item_skip_kernel<<<(n_items + 255) / 256, 256, 0, st>>>(rooms, items, n_items, pos_src, pos_rcv, skip);
-    return cudaGetLastError();
+    return launch_after(item_skip_kernel, (n_items + 255) / 256, 256, 0, st, rooms, items, n_items, pos_src, pos_rcv, skip);
 }
 
 // Sum of the partial segments of each group, parts in increasing order (the result
 // does not depend on which block computed which part).
 __global__ void partial_reduce_kernel(const PartGroup *groups, int n_groups, const float *part, float *out) {
+    after_previous();
     const int g = blockIdx.y;
     if (g >= n_groups) return;
     const PartGroup G = groups[g];
@@ -944,8 +945,7 @@ cudaError_t partial_reduce_launch(const PartGroup *groups, int n_groups, int max
     if (n_groups <= 0 || max_len <= 0) return cudaSuccess;
     if (n_groups > 65535) return cudaErrorInvalidValue;
     dim3 grid((unsigned)((max_len + 255) / 256), (unsigned)n_groups);
-    partial_reduce_kernel<<<grid, 256, 0, st>>>(groups, n_groups, part, out);
-    return cudaGetLastError();
+    return launch_after(partial_reduce_kernel, grid, 256, 0, st, groups, n_groups, part, out);
 }
 
 }  // namespace gpurir

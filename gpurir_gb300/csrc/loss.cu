@@ -6,7 +6,7 @@
 // and writes the gradient the adjoint kernel consumes; its last block to finish
 // adds the per-block partial sums in a fixed order (deterministic).
 // gpuRIR has no counterpart (it is not differentiable).
-#include <cuda_runtime.h>
+#include "launch.cuh"
 
 namespace gpurir {
 
@@ -33,6 +33,7 @@ __global__ void __launch_bounds__(kLossThreads) l2_grad_kernel(const float *__re
                                                                double *partial, float *__restrict__ loss, int *done) {
     __shared__ double red[kLossThreads / 32];
     __shared__ int last;
+    after_previous();
     const float two_s = 2.0f * scale;
     float acc = 0.0f;
     const long stride = (long)gridDim.x * kLossThreads;
@@ -81,8 +82,7 @@ cudaError_t l2_grad_launch(const float *y, const float *t, long n, float scale, 
                            float *loss, int *done, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
     const int blocks = l2_grad_blocks(n);
-    l2_grad_kernel<<<blocks, kLossThreads, 0, st>>>(y, t, n, scale, g, partial, loss, done);
-    return cudaGetLastError();
+    return launch_after(l2_grad_kernel, blocks, kLossThreads, 0, st, y, t, n, scale, g, partial, loss, done);
 }
 
 }  // namespace gpurir

@@ -43,6 +43,7 @@ __device__ __forceinline__ void clear_counters(int *ctl) {
 }
 
 __global__ void room_beta_kernel(RoomDesc *rooms, int n_rooms, const float *beta, int *ctl) {
+    after_previous();
     clear_counters(ctl);
     if ((int)blockIdx.x < n_rooms) room_beta_kernel_body(rooms, blockIdx.x, beta);
 }
@@ -53,6 +54,7 @@ __global__ void room_beta_kernel(RoomDesc *rooms, int n_rooms, const float *beta
 __global__ void room_beta_skip_kernel(RoomDesc *rooms, int n_rooms, const float *beta, const IsmItem *items,
                                       int n_items, const float *pos_src, const float *pos_rcv,
                                       unsigned char *skip, int *ctl) {
+    after_previous();
     clear_counters(ctl);
     if ((int)blockIdx.x < n_rooms) {
         if (threadIdx.x < 32) room_beta_kernel_body(rooms, blockIdx.x, beta);
@@ -76,14 +78,13 @@ cudaError_t room_beta_skip_launch(RoomDesc *rooms, int n_rooms, const float *bet
                                   int *ctl, cudaStream_t st) {
     const int blocks = n_rooms + (n_items + 255) / 256;
     if (blocks <= 0) return cudaSuccess;
-    room_beta_skip_kernel<<<blocks, 256, 0, st>>>(rooms, n_rooms, beta, items, n_items, pos_src, pos_rcv, skip, ctl);
-    return cudaGetLastError();
+    return launch_after(room_beta_skip_kernel, blocks, 256, 0, st, rooms, n_rooms, beta, items, n_items, pos_src, pos_rcv,
+                        skip, ctl);
 }
 
 cudaError_t room_beta_launch(RoomDesc *rooms, int n_rooms, const float *beta, int *ctl, cudaStream_t st) {
     if (n_rooms <= 0) return cudaSuccess;
-    room_beta_kernel<<<n_rooms, 32, 0, st>>>(rooms, n_rooms, beta, ctl);
-    return cudaGetLastError();
+    return launch_after(room_beta_kernel, n_rooms, 32, 0, st, rooms, n_rooms, beta, ctl);
 }
 
 }  // namespace gpurir

@@ -28,6 +28,7 @@ struct TailLaunch {
 };
 
 __global__ void __launch_bounds__(kTailThreads) tail_kernel(TailLaunch P) {
+    after_previous();
     const int rir = blockIdx.x;
     if (rir >= P.n_rir) return;
     const IsmItem it = P.rirs[rir];
@@ -91,8 +92,7 @@ cudaError_t tail_launch(const RoomDesc *rooms, const IsmItem *rirs, int n_rir, i
     const long chunks = ((long)max_n_diff + kTailChunk - 1) / kTailChunk;
     if (chunks > 65535) return cudaErrorInvalidValue;
     dim3 grid(n_rir, (unsigned)chunks);
-    tail_kernel<<<grid, kTailThreads, 0, st>>>(p);
-    return cudaGetLastError();
+    return launch_after(tail_kernel, grid, kTailThreads, 0, st, p);
 }
 
 // One thread: the call offset of a captured graph advances by one per replay.
