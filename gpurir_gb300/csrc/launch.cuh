@@ -18,6 +18,14 @@ __device__ __forceinline__ void after_previous() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// A pointer whose read-only loads (__ldg, const __restrict__) must not be moved before the wait:
+// the compiler may take such loads for free of any order, but not ahead of the pointer they use.
+template <class T>
+__device__ __forceinline__ T *after_wait(T *p) {
+    asm volatile("" : "+l"(p));
+    return p;
+}
+
 template <class... P, class... A>
 inline cudaError_t launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
     cudaLaunchAttribute attr;

@@ -34,6 +34,8 @@ __global__ void __launch_bounds__(kLossThreads) l2_grad_kernel(const float *__re
     __shared__ double red[kLossThreads / 32];
     __shared__ int last;
     after_previous();
+    y = after_wait(y);
+    t = after_wait(t);
     const float two_s = 2.0f * scale;
     float acc = 0.0f;
     const long stride = (long)gridDim.x * kLossThreads;
