@@ -612,6 +612,9 @@ __device__ __forceinline__ void load_packed(const float *__restrict__ x, int len
 template <int M>
 __global__ void __launch_bounds__(M / 16, 16384 / M) segment_spectra_reg_kernel(
         const float *__restrict__ seg, int P, int S, const float2 *__restrict__ W, float2 *__restrict__ Sg) {
+    after_previous();
+    seg = after_wait(seg);
+    W = after_wait(W);
     constexpr int T = M / 16;
     extern __shared__ __align__(16) float2 sm[];
     float2 *buf = sm;
@@ -746,6 +749,10 @@ template <int M, int ROWS>
 __global__ void __launch_bounds__(M / 16, (16384 / M / ROWS > 0 ? 16384 / M / ROWS : 1)) rir_conv_reg_kernel(
         const float *__restrict__ rir, int P, int R, int L, int S, const float2 *__restrict__ W,
         const float2 *__restrict__ Sg, float *__restrict__ out, long out_ld) {
+    after_previous();
+    rir = after_wait(rir);
+    W = after_wait(W);
+    Sg = after_wait(Sg);
     constexpr int T = M / 16, BS = M + M / 16;
     extern __shared__ __align__(16) float2 sm[];
     float2 *buf = sm;   // ROWS buffers of pad16(M) elements
@@ -866,8 +873,7 @@ static cudaError_t launch_reg_conv_rows(const float *rir, int P, int R, int L, i
         blocks = std::max(1, per_sm) * std::max(1, sms);
     }
     const int grid = std::min((P * R + ROWS - 1) / ROWS, blocks);
-    rir_conv_reg_kernel<M, ROWS><<<grid, M / 16, smem, st>>>(rir, P, R, L, S, W, Sg, out, out_ld);
-    return cudaGetLastError();
+    return launch_after(rir_conv_reg_kernel<M, ROWS>, grid, M / 16, smem, st, rir, P, R, L, S, W, Sg, out, out_ld);
 }
 
 // Rows per block from the tuning table (1: more blocks per SM; 2: twiddles and
@@ -898,6 +904,8 @@ static cudaError_t launch_reg_conv(const float *rir, int P, int R, int L, int S,
 
 // g [n_out][R] float64 -> gt [R][n_out] float32 (rows the FFT kernels read contiguously)
 __global__ void grad_transpose_kernel(const double *__restrict__ g, long n_out, int R, float *__restrict__ gt) {
+    after_previous();
+    g = after_wait(g);
     const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n_out) return;
     for (int r = 0; r < R; r++) gt[(long)r * n_out + t] = (float)g[t * R + r];
@@ -1172,6 +1180,9 @@ __device__ __forceinline__ void blk_inverse(float2 (&v)[16], float2 *buf, const 
 // 1 / 2048, in bin order.
 __global__ void __launch_bounds__(kBlkThreads) blk_spectra_kernel(const float *__restrict__ seg, int P, int S,
                                                                   const float2 *__restrict__ W, float2 *__restrict__ X) {
+    after_previous();
+    seg = after_wait(seg);
+    W = after_wait(W);
     __shared__ __align__(16) float2 buf[kBlk + kBlk / 16];
     __shared__ float2 tw[kBlkTw * kBlkThreads];
     const int j = threadIdx.x;
@@ -1198,6 +1209,13 @@ __global__ void __launch_bounds__(kBlkThreads, kBlkPerSm) traj_adjoint_blk_kerne
         const float *__restrict__ rir, int P, int R, int L, int S, int B, int n_pair, int runs, int run_pairs,
         const float2 *__restrict__ W, const float2 *__restrict__ X, float *__restrict__ grad_rir,
         float *__restrict__ part) {
+    after_previous();
+    gt = after_wait(gt);
+    w_ini = after_wait(w_ini);
+    w_len = after_wait(w_len);
+    rir = after_wait(rir);
+    W = after_wait(W);
+    X = after_wait(X);
     extern __shared__ __align__(16) float2 sm[];
     float2 *buf = sm, *tw = buf + kBlk + kBlk / 16;
     float2 *acc = tw + kBlkTw * kBlkThreads;   // [kBlk] this run's sum of G conj(H): entry 128 i + j is thread j's
@@ -1263,6 +1281,10 @@ __global__ void __launch_bounds__(kBlkThreads, kBlkPerSm) traj_adjoint_blk_kerne
 // dL/dx of each point: its runs' parts in order.
 __global__ void blk_sum_kernel(const float *__restrict__ part, const int *__restrict__ w_ini,
                                const int *__restrict__ w_len, int P, int S, int runs, float *__restrict__ grad_sig) {
+    after_previous();
+    part = after_wait(part);
+    w_ini = after_wait(w_ini);
+    w_len = after_wait(w_len);
     const int p = blockIdx.y, t = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= P || t >= w_len[p]) return;
     float a = 0.0f;
@@ -1299,21 +1321,23 @@ cudaError_t traj_adjoint_blk_launch(const double *g, long n_out, const int *w_in
                                     float *gt, float *work, float *grad_rir, float *grad_sig, cudaStream_t st) {
     float2 *X = reinterpret_cast<float2 *>(work);
     float *part = grad_sig ? work + (size_t)2 * P * kBlk : nullptr;
-    grad_transpose_kernel<<<(unsigned)((n_out + 255) / 256), 256, 0, st>>>(g, n_out, R, gt);
+    cudaError_t e = launch_after(grad_transpose_kernel, (unsigned)((n_out + 255) / 256), 256, 0, st, g, n_out, R, gt);
+    if (e != cudaSuccess) return e;
     const size_t smem = (size_t)(2 * kBlk + kBlk / 16 + kBlkTw * kBlkThreads) * sizeof(float2);
     static bool attr = false;
     if (!attr) {
-        cudaError_t e = cudaFuncSetAttribute(traj_adjoint_blk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        e = cudaFuncSetAttribute(traj_adjoint_blk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
         attr = true;
     }
-    if (grad_rir) blk_spectra_kernel<<<std::min(P, b.grid), kBlkThreads, 0, st>>>(seg, P, S, W, X);
-    traj_adjoint_blk_kernel<<<b.grid, kBlkThreads, smem, st>>>(gt, n_out, w_ini, w_len, rir, P, R, L, S, b.B, b.n_pair, b.runs,
-                                                            b.run_pairs, W, X, grad_rir, part);
+    if (grad_rir) e = launch_after(blk_spectra_kernel, std::min(P, b.grid), kBlkThreads, 0, st, seg, P, S, W, X);
+    if (e != cudaSuccess) return e;
+    e = launch_after(traj_adjoint_blk_kernel, b.grid, kBlkThreads, smem, st, gt, n_out, w_ini, w_len, rir, P, R, L, S, b.B, b.n_pair,
+                     b.runs, b.run_pairs, W, X, grad_rir, part);
+    if (e != cudaSuccess) return e;
     if (grad_sig)
-        blk_sum_kernel<<<dim3((unsigned)((S + 127) / 128), (unsigned)P), 128, 0, st>>>(part, w_ini, w_len, P, S, b.runs,
-                                                                                        grad_sig);
-    return cudaGetLastError();
+        e = launch_after(blk_sum_kernel, dim3((unsigned)((S + 127) / 128), (unsigned)P), 128, 0, st, part, w_ini, w_len, P, S, b.runs, grad_sig);
+    return e;
 }
 
 template <int M>
@@ -1363,6 +1387,7 @@ cudaError_t traj_adjoint_launch(const double *g, long n_out, const int *w_ini, c
 // Compensated FP32 sum (two-sum), written as float64.
 __global__ void ola_kernel(const float *conv, long conv_ld, const int *w_ini, const int *w_len, int P,
                            int R, int L, long n_out, int uni_w, double *out) {
+    after_previous();
     const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;   // consecutive t: coalesced reads
     const int r = blockIdx.y;
     if (t >= n_out) return;
@@ -1456,8 +1481,7 @@ static cudaError_t launch_reg_spectra(const float *seg, int P, int S, const floa
         if (e != cudaSuccess) return e;
         blocks = std::max(1, per_sm) * std::max(1, sms);
     }
-    segment_spectra_reg_kernel<M><<<std::min(P, blocks), M / 16, smem, st>>>(seg, P, S, W, Sg);
-    return cudaGetLastError();
+    return launch_after(segment_spectra_reg_kernel<M>, std::min(P, blocks), M / 16, smem, st, seg, P, S, W, Sg);
 }
 
 cudaError_t segment_spectra_launch(const float *seg, int P, int S, int M, const float2 *W, float2 *Sg,
@@ -1497,8 +1521,7 @@ cudaError_t ola_launch(const float *conv, long conv_ld, const int *w_ini, const 
     if (n_out <= 0 || R <= 0) return cudaSuccess;
     if (R > 65535) return cudaErrorInvalidValue;
     dim3 grid((unsigned)((n_out + 255) / 256), (unsigned)R);
-    ola_kernel<<<grid, 256, 0, st>>>(conv, conv_ld, w_ini, w_len, P, R, L, n_out, uni_w, out);
-    return cudaGetLastError();
+    return launch_after(ola_kernel, grid, 256, 0, st, conv, conv_ld, w_ini, w_len, P, R, L, n_out, uni_w, out);
 }
 
 }  // namespace gpurir
