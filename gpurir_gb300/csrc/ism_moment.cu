@@ -44,8 +44,8 @@
 // cells, 3.6 wavefronts; an FP32 atomicAdd takes 9.3 cycles) where images are many -- the
 // load pipe is at 77 % on 128 rooms -- and issue with the phases' barriers where they are few
 // (56 % of the slots on the array).  Per launch, ism_forward.cu and this kernel: one dense RIR of
-// 6 million images 531 and 98 us, 64 x 32 array 490 and 327, 128 rooms 2620 and 617, 15 RIRs at
-// 48 kHz 87 and 40.  (Other ways that were built first: a counting sort by cell with one
+// 6 million images 531 and 91 us, 64 x 32 array 490 and 321, 128 rooms 2680 and 606, 15 RIRs at
+// 48 kHz 87 and 38.  (Other ways that were built first: a counting sort by cell with one
 // thread per cell adding in image order needed 8 barriers per 1024 images and ran at 228
 // cycles per 32 images and SM, against 90 here.)
 #include <algorithm>
