@@ -231,6 +231,12 @@ class Simulator:
         _lib.check(self._L.gpurir_last_launch_count(self._h, ctypes.byref(v)), "last_launch_count")
         return v.value
 
+    def last_moment_rirs(self):
+        """RIRs whose early part the last simulate call computed by fractional-delay moments."""
+        v = ctypes.c_longlong()
+        _lib.check(self._L.gpurir_last_moment_rirs(self._h, ctypes.byref(v)), "last_moment_rirs")
+        return v.value
+
     def set_profiling(self, on=True):
         _lib.check(self._L.gpurir_set_profiling(self._h, int(bool(on))), "set_profiling")
 

@@ -147,6 +147,7 @@ struct gpurir_sim {
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     bool ev_ism = false, ev_tail = false;
     int last_launches = 0;        // kernels the last simulate call launched
+    long last_moment_rirs = 0;    // RIRs whose early part it left to the moment kernel
     // The plan of the last simulate call, reused by a call with the same room shapes
     // (sizes, image counts, lengths, source/receiver counts: what the work items depend
     // on); its items stay on the device while ws_gen == the generation they were
@@ -961,7 +962,10 @@ static int enqueue_kernels(gpurir_sim *s, const Plan &P, const char *d, const La
     ta.env_out = reinterpret_cast<float *>(const_cast<char *>(d) + L.o_env);
     ta.fuse = 1;
     ta.pre = tail_pre;
-    if (record) s->last_launches = (P.grid > 0 ? 1 : 0);
+    if (record) {
+        s->last_launches = (P.grid > 0 ? 1 : 0);
+        s->last_moment_rirs = P.mom && P.grid > 0 ? M : 0;
+    }
     unsigned char *skip = nullptr;
     if (P.grid > 0 && P.skip_flags) {   // segments no image may reach: flags at the current positions
         skip = reinterpret_cast<unsigned char *>(const_cast<char *>(d) + L.o_skip);
@@ -1341,6 +1345,12 @@ extern "C" int gpurir_set_profiling(gpurir_sim *s, int on) {
 extern "C" int gpurir_last_launch_count(gpurir_sim *s, int *kernels) {
     if (!s || !kernels) return fail(GPURIR_ERR_INVALID, "NULL argument");
     *kernels = s->last_launches;
+    return GPURIR_OK;
+}
+
+extern "C" int gpurir_last_moment_rirs(gpurir_sim *s, long long *rirs) {
+    if (!s || !rirs) return fail(GPURIR_ERR_INVALID, "NULL argument");
+    *rirs = s->last_moment_rirs;
     return GPURIR_OK;
 }
 

@@ -345,6 +345,11 @@ int gpurir_host_free(void *ptr);
  * the reference. */
 int gpurir_last_launch_count(gpurir_sim *sim, int *kernels);
 
+/* Number of RIRs whose early part the last simulate call on `sim` computed by
+ * fractional-delay moments; the others were summed tap by tap.  No counterpart in
+ * the reference. */
+int gpurir_last_moment_rirs(gpurir_sim *sim, long long *rirs);
+
 /* Kernel timing: when on, each simulate call records CUDA events on its
  * stream around the ISM kernel and the tail kernel; gpurir_last_timing waits
  * for them and returns the two durations in ms (0 for a kernel not launched).
