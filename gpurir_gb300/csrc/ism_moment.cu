@@ -4,7 +4,9 @@
 // (src/gpuRIR_cuda.cu:110-121).  ism_forward.cu adds each image's Tw taps one by one;
 // this kernel separates them.  Time is cut into cells of two samples; with tau = n + u, n
 // the cell's centre and u in [-1, 1], each tap W(kappa - u), kappa = t - n, is a smooth
-// function of u and a polynomial of degree 13 reproduces all of them (2e-8 relative L2):
+// function of u and a polynomial of degree 13 reproduces all of them (3 to 4e-8 relative L2, 6e-8 at
+// the shortest windows; of the images whose window ends in the middle of a cell 5e-8 from 80 samples
+// of window on, up to 2.1e-7 below, all of it in the last tap):
 //   y[t] = sum over cells n, sum_j c_j(t - n) A_j[n],   A_j[n] = sum over the cell's images of a T_j(u)
 // with T_j the Chebyshev polynomials.  An image then costs its geometry and fourteen
 // multiply-adds instead of Tw taps, and a sample costs a fixed filter whatever the number
@@ -29,23 +31,24 @@
 //      lane) and a range of taps; the warps' parts are added in order.
 //
 // The sums are integers, so that their order -- whichever warp comes first -- does not
-// change a bit: a moment is scaled by a power of two (from a bound on the segment's
-// amplitudes) to at most 2^20, rounded to an integer, and its remainder to 2^-20 of that to
-// a second one (both roundings by the addition of 1.5 2^23, whose bits are added up as they
-// are and removed by the count): 41 bits below the segment's largest amplitude.  T_8 to
-// T_13, whose taps' coefficients are below 2e-3, have the first integer only.  Cells of up to
-// 448 images need fewer guard bits and share words (kMPSums below): 17 words a cell instead
-// of 23, 28 to 31 bits below the bound, which follows the attenuation of each segment.  An
-// image too near for the bound (below 5 cm) goes into a short list and is added in FP32 in
-// a fixed order; a segment with more of those, or with cells of more images than the
-// integers hold, is done again with bounds that fit.
+// change a bit: a moment is scaled by a power of two (from a bound on the amplitudes) to at most
+// 2^20, rounded to an integer, and its remainder to 2^-20 of that to a second one (both
+// roundings by the addition of 1.5 2^23, whose bits are added up as they are and removed by the
+// count): 41 bits below the bound.  T_8 to T_13, whose taps' coefficients are below 2e-3, have
+// the first integer only.  Cells of up to 448 images need fewer guard bits and share words
+// (kMPSums below): 17 words a cell instead of 23, 28 to 31 bits below the bound.  Either way an
+// image adds an error of about 2e-10 of the bound.  Where a segment's loudest image is far above
+// its quietest samples -- most first segments, any with dull walls -- the bound is that of every
+// eight cells by themselves (16 samples, fewer than an image's taps reach), from a first pass
+// over the images, so that the error stays below FP32's own.  A segment with cells of more
+// images than the integers hold is done again with bounds that fit.
 //
 // What bounds it: the shared-memory atomics of the image loop (2.7 cycles per warp at random
 // cells, 3.6 wavefronts; an FP32 atomicAdd takes 9.3 cycles) where images are many -- the
 // load pipe is at 77 % on 128 rooms -- and issue with the phases' barriers where they are few
 // (56 % of the slots on the array).  Per launch, ism_forward.cu and this kernel: one dense RIR of
-// 6 million images 531 and 91 us, 64 x 32 array 490 and 321, 128 rooms 2680 and 606, 15 RIRs at
-// 48 kHz 87 and 38.  (Other ways that were built first: a counting sort by cell with one
+// 6 million images 531 and 95 us, 64 x 32 array 490 and 322, 128 rooms 2680 and 670, 15 RIRs at
+// 48 kHz 87 and 37 (with one scale per segment 90, 321, 625 and 37).  (Other ways that were built first: a counting sort by cell with one
 // thread per cell adding in image order needed 8 barriers per 1024 images and ran at 228
 // cycles per 32 images and SM, against 90 here.)
 #include <algorithm>
@@ -85,7 +88,9 @@ constexpr int kMSums = 4 * kMTwo + 2 * (kMPairs - kMTwo) + 1;   // integers per 
 constexpr int kMPTwo = 4, kMPSums = 3 * kMPTwo + 2 + 3;
 constexpr int kMPSpan = 21, kMPCount = 10, kMPMinBits = 6, kMPMaxBits = 9;
 static_assert(kMPairs == 7, "the packed words are laid out for fourteen moments");
-constexpr int kMLoud = 32;                     // images of a segment above the bound of its scale
+constexpr int kMScale = 3;                     // log2 of the cells that share a scale
+constexpr int kMScales = kMomCells >> kMScale; // at most
+static_assert(kMScales + kMomCells / 32 <= kMomSmall && kMomSmallCells <= kMomCells, "a thread for each scale and word of bits");
 constexpr float kMMagic = 12582912.0f;         // 1.5 2^23
 constexpr int kMMagicBits = 0x4b400000;
 
@@ -114,7 +119,8 @@ struct MomSmem {
     float4 *rows;             // [rows] rho^2 hi, lo, attenuation, m0 | m1 << 16
     int2 *range;              // [rows] first image, za | na << 9 | zb << 18
     unsigned short *group;    // [groups] row of a group's first image
-    float4 *loud;             // [kMLoud] a, u, cell
+    int *scale;               // [kMScales] bits of the loudest image of eight cells; then of their scale
+    unsigned *bad;            // [kMomCells / 32] cells with an image of no finite amplitude, as bits
     MomCtx *ctx;              // [2]
     int *red;                 // scan scratch [32], control words [16]
     float4 *tab;              // [2][axis_cap] per-axis tables (or in global memory)
@@ -124,7 +130,7 @@ __host__ __device__ inline size_t mom_align16(size_t x) { return (x + 15) & ~(si
 
 // Byte offsets of the arrays of MomSmem, in its order; returns the total.
 template <class Cfg>
-__host__ __device__ inline size_t mom_layout(int n_quads, int axis_cap, size_t o[9]) {
+__host__ __device__ inline size_t mom_layout(int n_quads, int axis_cap, size_t o[10]) {
     const size_t sums = (size_t)kMSums * Cfg::stride * sizeof(int);
     const size_t filt = (size_t)kMBasis * Cfg::stride * sizeof(float2) + (size_t)Cfg::warps * 512 * sizeof(float);
     size_t b = 0;
@@ -133,10 +139,11 @@ __host__ __device__ inline size_t mom_layout(int n_quads, int axis_cap, size_t o
     o[2] = b; b = b + Cfg::rows * sizeof(float4);
     o[3] = b; b = b + Cfg::rows * sizeof(int2);
     o[4] = b; b = b + Cfg::groups * sizeof(unsigned short);
-    o[5] = b; b = b + kMLoud * sizeof(float4);
-    o[6] = b; b = mom_align16(b + 2 * sizeof(MomCtx));
-    o[7] = b; b = mom_align16(b + 48 * sizeof(int));
-    o[8] = b; b += axis_cap <= kMomTabSmem ? 2 * (size_t)axis_cap * sizeof(float4) : 0;
+    o[5] = b; b = b + kMScales * sizeof(int);
+    o[6] = b; b = b + kMomCells / 32 * sizeof(int);
+    o[7] = b; b = mom_align16(b + 2 * sizeof(MomCtx));
+    o[8] = b; b = mom_align16(b + 48 * sizeof(int));
+    o[9] = b; b += axis_cap <= kMomTabSmem ? 2 * (size_t)axis_cap * sizeof(float4) : 0;
     return b;
 }
 
@@ -146,8 +153,8 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
     return r;
 }
 
-// Exclusive block scan of one int per thread; `tot` is the block's sum.  red: 32 ints
-// (two calls in a row use different halves of the scratch, so one barrier each).
+// Exclusive block scan of one int per thread; `tot` is the block's sum.  red: WARPS ints, free
+// again at the caller's next barrier.
 template <int WARPS>
 __device__ __forceinline__ int block_scan(int v, int *red, int &tot) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -352,33 +359,6 @@ __device__ __forceinline__ void image_moments(float a, float u, Put put) {
     }
 }
 
-// The order in which a cell's loud images are added: by u, then by a (images equal in
-// both are the same).
-__device__ __forceinline__ bool record_less(float2 p, float2 q) { return p.y < q.y || (p.y == q.y && p.x < q.x); }
-// Adds the loud images of a cell in that order (a few images of a few cells).
-__device__ __noinline__ void add_loud(float2 (&A)[kMPairs], const float4 *loud, int n, int cell) {
-    float2 done = make_float2(0.0f, -8.0f);   // the images up to here are added
-    for (;;) {
-        float2 best = make_float2(0.0f, 8.0f);
-        int same = 0;
-        for (int k = 0; k < n; k++) {
-            const float4 v = loud[k];
-            const float2 r = make_float2(v.x, v.y);
-            if (__float_as_int(v.z) != cell || !record_less(done, r)) continue;
-            if (record_less(r, best)) {
-                best = r;
-                same = 1;
-            } else if (r.x == best.x && r.y == best.y) {
-                same++;
-            }
-        }
-        if (same == 0) return;
-        for (int k = 0; k < same; k++)
-            image_moments(best.x, best.y, [&](int p, float2 v) { A[p] = add2_rn(A[p], v); });
-        done = best;
-    }
-}
-
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS, MomCfg<THREADS>::blocks) ism_moment_kernel(const __grid_constant__ MomLaunch P) {
     using Cfg = MomCfg<THREADS>;
@@ -386,23 +366,25 @@ __global__ void __launch_bounds__(THREADS, MomCfg<THREADS>::blocks) ism_moment_k
     extern __shared__ __align__(16) unsigned char smem_raw[];
     MomSmem s;
     {
-        size_t o[9];
+        size_t o[10];
         mom_layout<Cfg>(P.n_quads, P.axis_cap, o);
         s.sum = reinterpret_cast<int *>(smem_raw + o[0]);
         s.coef = reinterpret_cast<float2 *>(smem_raw + o[1]);
         s.rows = reinterpret_cast<float4 *>(smem_raw + o[2]);
         s.range = reinterpret_cast<int2 *>(smem_raw + o[3]);
         s.group = reinterpret_cast<unsigned short *>(smem_raw + o[4]);
-        s.loud = reinterpret_cast<float4 *>(smem_raw + o[5]);
-        s.ctx = reinterpret_cast<MomCtx *>(smem_raw + o[6]);
-        s.red = reinterpret_cast<int *>(smem_raw + o[7]);
-        s.tab = P.axis_cap <= kMomTabSmem ? reinterpret_cast<float4 *>(smem_raw + o[8])
+        s.scale = reinterpret_cast<int *>(smem_raw + o[5]);
+        s.bad = reinterpret_cast<unsigned *>(smem_raw + o[6]);
+        s.ctx = reinterpret_cast<MomCtx *>(smem_raw + o[7]);
+        s.red = reinterpret_cast<int *>(smem_raw + o[8]);
+        s.tab = P.axis_cap <= kMomTabSmem ? reinterpret_cast<float4 *>(smem_raw + o[9])
                                         : P.axis_tab + (size_t)(2 * blockIdx.x) * P.axis_cap;
     }
     float2 *basis = reinterpret_cast<float2 *>(s.sum);                 // [kMBasis][kMStride]
     float *part = reinterpret_cast<float *>(basis + kMBasis * kMStride);  // filter parts
-    int *ctl = s.red + 32;   // [0] most images of a cell, [1] last cell with an image, [2] loud images,
-                             // [3..8] bounds of |attenuation| along the axes, [9] images not counted in a cell
+    int *ctl = s.red + 32;   // [0] most images of a cell, [1] last cell with an image, [2] a cell is bad,
+                             // [3] images not counted in a cell, [4..9] bounds of |attenuation| along the axes, [10, 11]
+                             // an image's attenuation at the segment's ends
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const unsigned le_mask = 0xffffffffu >> (31 - lane);
     for (int i = tid; i < 8 * P.n_quads; i += kMThreads) s.coef[i] = P.coef[i];
@@ -469,6 +451,7 @@ __global__ void __launch_bounds__(THREADS, MomCfg<THREADS>::blocks) ism_moment_k
             // (in registers: the atomics might alias the context, so that it would be read again per image)
             const int kind = R.spkr | R.mic << 8 | (R.ref_delay != 0) << 16;
             const ff k_samples = {R.kh, R.kl};
+            const float k_scale = R.kh * (0.5f / (1 << kMScale)), g0 = (float)cell0 * (0.5f / (1 << kMScale));   // groups of cells
             const int batch = min(Cfg::rows, 32 * Cfg::groups / N2);   // rows at once: their images fill the groups at most
             // mean images per cell at the segment's end: a room's volume holds one; cells with few
             // have packed sums
@@ -476,58 +459,94 @@ __global__ void __launch_bounds__(THREADS, MomCfg<THREADS>::blocks) ism_moment_k
             int bits = kMPMinBits;
             while (bits < kMPMaxBits && 4.0f * mean + 24.0f > (float)(7 << bits >> 3)) bits++;
             bool packed = 2.0f * mean + 24.0f <= (float)(7 << bits >> 3);
-            float unit;        // value of one step of a sum's first integer
             int shift = 0;     // bits given up to hold more images per cell
-            for (int round = 0;;) {
+            int span = 0;      // log2 of the steps that cover an amplitude, of the scales at hand
+            int n_rows = 0, n_img = 0;
+            bool rows_ready = false;   // a segment's only batch of rows stays in place
+            for (;;) {
                 const int words = packed ? kMPSums : kMSums;
                 for (int a = warp; a < words; a += kMWarps)
                     for (int i = lane; 4 * i < nbe; i += 32)
                         reinterpret_cast<int4 *>(s.sum + a * kMStride)[i] = make_int4(0, 0, 0, 0);
-                if (warp < 3) {   // largest |attenuation| along one axis, and beyond d_lo / sqrt(3)
-                    int a2, b2;
-                    axis_range(N2, inv_L2, C.ov[2], C.pos[5], d_hi, a2, b2);
-                    const int lo = warp == 0 ? a0 : (warp == 1 ? N0 + a1 : N0 + N1 + a2);
-                    const int hi = warp == 0 ? a0 + (W1 > 0 ? n_box / W1 : 0) : (warp == 1 ? N0 + a1 + W1 : N0 + N1 + b2);
-                    const float far2 = 0.3333f * dlo2;
-                    int full = 0, far = 0;
-                    for (int i = lo + lane; i < hi; i += 32) {
-                        const int w = __float_as_int(fabsf(tab[i].w));
-                        full = max(full, w);
-                        if (!(tab[i].x < far2)) far = max(far, w);
+                if (tid < 4) ctl[tid] = tid == 1 ? -1 : 0;
+                const int spans = packed ? kMPSpan : 20 - shift;
+                const float most = __int_as_float((127 + spans) << 23);
+                const float fine = packed ? __int_as_float((127 + 16 - bits) << 23) : most;   // steps of the second integer in one of the first
+                if (span == 0) {
+                    if (tid < kMScales) s.scale[tid] = 0;
+                    else if (tid - kMScales < kMomCells / 32) s.bad[tid - kMScales] = 0;
+                    if (warp < 3) {   // largest |attenuation| along one axis, and beyond d_lo / sqrt(3)
+                        int a2, b2;
+                        axis_range(N2, inv_L2, C.ov[2], C.pos[5], d_hi, a2, b2);
+                        const int lo = warp == 0 ? a0 : (warp == 1 ? N0 + a1 : N0 + N1 + a2);
+                        const int hi = warp == 0 ? a0 + (W1 > 0 ? n_box / W1 : 0) : (warp == 1 ? N0 + a1 + W1 : N0 + N1 + b2);
+                        const float far2 = 0.3333f * dlo2;
+                        int full = 0, far = 0;
+                        for (int i = lo + lane; i < hi; i += 32) {
+                            const int w = __float_as_int(fabsf(tab[i].w));
+                            full = max(full, w);
+                            if (!(tab[i].x < far2)) far = max(far, w);
+                        }
+                        full = __reduce_max_sync(0xffffffffu, full);
+                        far = __reduce_max_sync(0xffffffffu, far);
+                        if (lane == 0) {
+                            ctl[4 + warp] = full;
+                            ctl[7 + warp] = far;
+                        }
+                    } else if (warp == 3) {   // images d_lo and d_hi away in no special direction: half of that along each axis
+                        const int axis = lane & 3;
+                        float att = 1.0f;
+                        if (lane < 8 && axis < 3) {
+                            const int N = R.nb[axis], c = N / 2;
+                            const int n = (int)fminf(0.5f * (lane < 4 ? d_lo : d_hi) * C.inv_L[axis], 1.0e6f) + (lane >> 2);
+                            const float4 *t = tab + (axis > 0 ? N0 : 0) + (axis > 1 ? N1 : 0);
+                            att = fminf(fabsf(t[max(c - n, 0)].w), fabsf(t[min(c + n, N - 1)].w));
+                        }
+                        att *= __shfl_xor_sync(0xffffffffu, att, 1);
+                        att *= __shfl_xor_sync(0xffffffffu, att, 2);
+                        if (lane == 0 || lane == 4) ctl[10 + (lane >> 2)] = __float_as_int(att);
                     }
-                    full = __reduce_max_sync(0xffffffffu, full);
-                    far = __reduce_max_sync(0xffffffffu, far);
-                    if (lane == 0) {
-                        ctl[3 + warp] = full;
-                        ctl[6 + warp] = far;
-                    }
-                } else if (warp == 3) {
-                    if (lane < 3) ctl[lane] = lane == 1 ? -1 : 0;
-                    if (lane == 3) ctl[9] = 0;
                 }
                 __syncthreads();
-                // scale: of an image at least d_lo away one component is d_lo / sqrt(3) at least, which bounds
-                // its attenuation (walls that amplify too), and amplitudes are at most that bound over
-                // 4 pi d with d the shell's inner radius or the nearest image's distance; at first images
-                // nearer than 5 cm are left to the loud list.  2^(e + 1) bounds them; the span of the steps
-                // (2^(20 - shift), 2^21 packed) covers that.
-                float att_max;
-                {
-                    const float f0 = __int_as_float(ctl[3]), f1 = __int_as_float(ctl[4]), f2 = __int_as_float(ctl[5]);
-                    att_max = fmaxf(fmaxf(__int_as_float(ctl[6]) * (f1 * f2), __int_as_float(ctl[7]) * (f0 * f2)),
-                                    __int_as_float(ctl[8]) * (f0 * f1));
+                // One scale for the segment where its loudest image is not far above an image at either end: of an
+                // image at least d_lo away one component is d_lo / sqrt(3) at least, which bounds its attenuation
+                // (walls that amplify too), and amplitudes are at most that bound over 4 pi d with d the shell's
+                // inner radius or the nearest image's distance.  An image's error of 2e-10 of that bound is then at
+                // most 3e-8 of the quiet ones.  Else every eight cells (16 samples) have a scale of their own, from
+                // the loudest of their images.  (With one scale always, 128 samples of a first segment were off by
+                // 2e-4 at 16 kHz and 0.15 at 8 kHz with walls of 0.1, by 2e-6 and 1.5e-4 with walls of 0.3; now 4e-7
+                // at most.  With a scale per eight cells always, 128 rooms take 887 us instead of 670.)
+                int uniform = 0;
+                bool quiet = false;
+                if (span == 0) {
+                    const float f0 = __int_as_float(ctl[4]), f1 = __int_as_float(ctl[5]), f2 = __int_as_float(ctl[6]);
+                    const float att_max = fmaxf(fmaxf(__int_as_float(ctl[7]) * (f1 * f2), __int_as_float(ctl[8]) * (f0 * f2)),
+                                                __int_as_float(ctl[9]) * (f0 * f1));
+                    const float first = sqrtf(__int_as_float(C.near2[0]) + __int_as_float(C.near2[1]) +
+                                              __int_as_float(C.near2[2])) * 0.999f;
+                    const float near = fmaxf(d_lo, first), peak = att_max * 1.001f / near;
+                    quiet = max(max(ctl[4], ctl[5]), ctl[6]) >= 0x7f800000 ||   // (a factor that is not finite)
+                            !(peak < 3.0e38f && peak * near <= 128.0f * __int_as_float(ctl[10]) &&
+                              peak * d_hi <= 128.0f * __int_as_float(ctl[11]));
+                    uniform = __float_as_int(peak);
                 }
-                const float first = sqrtf(__int_as_float(C.near2[0]) + __int_as_float(C.near2[1]) +
-                                          __int_as_float(C.near2[2])) * 0.999f;
-                const float near = fmaxf(fmaxf(d_lo, first), round == 0 ? 0.05f : 1.0e-12f);
-                const int e = (__float_as_int(att_max * 0.0797f / near) >> 23) - 127;
-                const int span = packed ? kMPSpan : 20 - shift;
-                const int k = min(max(span - 1 - e, -120), 120);
-                const float scale = __int_as_float((127 + k) << 23), most = __int_as_float((127 + span) << 23);
-                const float fine = packed ? __int_as_float((127 + 16 - bits) << 23) : most;   // steps of the second integer in one of the first
-                unit = __int_as_float((127 - k) << 23);
                 int placed = 0;
+                // twice over the images of a quiet segment: the loudest of every eight cells, by an estimate of
+                // distance and amplitude that is good to 1e-6; then the sums, at the scales that follow
+                for (int sums = !quiet; sums < 2; sums++) {
+                if (sums) {
+                    if (quiet) __syncthreads();   // peaks complete
+                    if (tid < kMScales) {   // 2^(e + 1) bounds the amplitudes of these eight cells; the steps' span covers that
+                        const int v = span > 0 || quiet ? s.scale[tid] : uniform;
+                        const int e = (__float_as_int(__int_as_float(v) * 0.0797f) >> 23) - 127;   // (1 / 4 pi, and room for rounding)
+                        s.scale[tid] = span == 0 ? (127 + min(max(spans - 1 - e, -120), 120)) << 23
+                                                 : v + (spans - span) * (1 << 23);
+                    }
+                    span = spans;
+                    if (rows_ready) __syncthreads();   // (else the rows' barriers come first)
+                }
                 for (int rbase = 0; rbase < my_rows; rbase += batch) {
+                    if (!rows_ready) {
                     // ---- one row per thread: its m2 ranges [za, ya) and [zb, yb)
                     int za = 0, ya = 0, zb = 0, yb = 0;
                     float4 row = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -553,8 +572,11 @@ __global__ void __launch_bounds__(THREADS, MomCfg<THREADS>::blocks) ism_moment_k
                         for (int g = (off + 31) >> 5; 32 * g < off + mine; g++) s.group[g] = (unsigned short)my_row;
                     }
                     __syncthreads();
+                    n_rows = total >> 20;
+                    n_img = total & 0xfffff;
+                    rows_ready = my_rows <= batch;
+                    }
                     // ---- images, 32 of the batch per warp at a time
-                    const int n_rows = total >> 20, n_img = total & 0xfffff;
                     for (int base = 32 * warp; base < n_img; base += 32 * kMWarps) {
                         const int r0 = s.group[base >> 5], idx = base + lane;
                         // rows that begin inside this group, as bits
@@ -566,6 +588,17 @@ __global__ void __launch_bounds__(THREADS, MomCfg<THREADS>::blocks) ism_moment_k
                         const int j = idx - rg.x, na = (rg.y >> 9) & 511;
                         const int m2 = j < na ? (rg.y & 511) + j : (rg.y >> 18) + (j - na);
                         const float4 t2 = tab[N0 + N1 + m2];
+                        if (!sums) {
+                            const float d2 = row.x + t2.x, rs = rsqrt_approx(d2), a = fabsf(row.z * t2.w) * rs;
+                            const float g = d2 * rs * k_scale, room = fmaf(g, 2e-6f, 0.002f);   // groups from sample 0, the estimate's error
+                            const float ga = floorf(g - g0 - room), gb = floorf(g - g0 + room);
+                            if (!(gb >= 0.0f && ga < (float)kMScales) || !(a < 3.0e38f)) continue;
+                            for (int k = max((int)ga, 0); k <= min((int)gb, kMScales - 1); k++) {
+                                int *peak = s.scale + k;
+                                if (__float_as_int(a) > *(volatile int *)peak) atomicMax(peak, __float_as_int(a));
+                            }
+                            continue;
+                        }
                         ff d2 = ff_add(ff{row.x, row.y}, ff{t2.x, t2.y});
                         float v0h = 0.0f, v1h = 0.0f;
                         const int m0 = __float_as_int(row.w) & 0xffff, m1 = __float_as_int(row.w) >> 16;
@@ -597,10 +630,10 @@ __global__ void __launch_bounds__(THREADS, MomCfg<THREADS>::blocks) ism_moment_k
                         const float u = (tau.hi - (2.0f * (mg - kMMagic) + 1.0f)) + tau.lo;
                         const int b = __float_as_int(mg) - kMMagicBits - (cell0 >> 1);
                         if (!(tau.hi < 4.0e6f) || b < 0 || b >= nb || amp == 0.0f) continue;
-                        const float q = amp * scale;   // exact
-                        if (!(fabsf(q) <= most)) {
-                            const int l = atomicAdd(&ctl[2], 1);
-                            if (l < kMLoud) s.loud[l] = make_float4(amp, u, __int_as_float(b), 0.0f);
+                        const float q = amp * __int_as_float(s.scale[b >> kMScale]);   // exact
+                        if (!(fabsf(q) <= most)) {   // (finite amplitudes are covered)
+                            atomicOr(&s.bad[b >> 5], 1u << (b & 31));
+                            ctl[2] = 1;
                             continue;
                         }
                         int *cell = s.sum + b;
@@ -639,6 +672,7 @@ __global__ void __launch_bounds__(THREADS, MomCfg<THREADS>::blocks) ism_moment_k
                         });
                     }
                 }
+                }
                 __syncthreads();   // sums complete
                 int n_max = 0, top = -1;
                 const int *count = s.sum + (packed ? 3 * kMPTwo + 3 : kMSums - 1) * kMStride;
@@ -646,29 +680,27 @@ __global__ void __launch_bounds__(THREADS, MomCfg<THREADS>::blocks) ism_moment_k
                     const int n = packed ? count[b] & ((1 << kMPCount) - 1) : count[b];
                     n_max = max(n_max, n);
                     placed -= n;
-                    if (n > 0) top = b;
+                    if (n > 0 || (ctl[2] && s.bad[b >> 5] >> (b & 31) & 1)) top = b;
                 }
-                for (int l = 0; l < min(ctl[2], kMLoud); l++) top = max(top, __float_as_int(s.loud[l].z));
                 n_max = __reduce_max_sync(0xffffffffu, n_max);
                 top = __reduce_max_sync(0xffffffffu, top);
                 placed = __reduce_add_sync(0xffffffffu, placed);
                 if (lane == 0) {
                     atomicMax(&ctl[0], n_max);
                     atomicMax(&ctl[1], top);
-                    atomicAdd(&ctl[9], placed);
+                    atomicAdd(&ctl[3], placed);
                 }
                 __syncthreads();
                 if (packed) {   // too many images in a cell, or more than its count holds: unpacked sums
-                    if (ctl[0] <= (7 << bits >> 3) && ctl[9] == 0 && ctl[2] <= kMLoud) break;
+                    if (ctl[0] <= (7 << bits >> 3) && ctl[3] == 0) break;
                     packed = false;
                 } else {        // a cell's sums hold 2^(11 + shift) images
-                    if (round > 0 || (ctl[0] < 2048 && ctl[2] <= kMLoud)) break;
+                    if (ctl[0] >> (11 + shift) == 0) break;
                     while (ctl[0] >> (11 + shift)) shift++;
-                    round++;
                 }
                 __syncthreads();
             }
-            const int n_loud = ctl[2];
+            const bool any_bad = ctl[2] != 0;
             act = ctl[1] >= 0 ? min((ctl[1] >> 8) + 1, tiles) : 0;
             // ---- sums -> basis, each cell by one thread
             const float fine = __int_as_float((127 - (packed ? 16 - bits : 20 - shift)) << 23);
@@ -681,7 +713,8 @@ __global__ void __launch_bounds__(THREADS, MomCfg<THREADS>::blocks) ism_moment_k
                 const int *sum = s.sum + b;
                 const int tc = b < nbe ? sum[(packed ? 3 * kMPTwo + 3 : kMSums - 1) * kMStride] : 0;
                 const int n = packed ? tc & ((1 << kMPCount) - 1) : tc;
-                if (b >= nbe || (n == 0 && n_loud == 0)) continue;
+                if (b >= nbe || (n == 0 && !any_bad)) continue;
+                const float unit = __int_as_float((254 << 23) - s.scale[b >> kMScale]);   // of a step, one over the scale
                 const int bias = n * kMMagicBits;   // (modulo 2^32, as the sums)
                 float2 A[kMPairs];
                 if (packed) {
@@ -713,11 +746,7 @@ __global__ void __launch_bounds__(THREADS, MomCfg<THREADS>::blocks) ism_moment_k
                         A[p].y *= unit;
                     }
                 }
-                if (n_loud > kMLoud) {   // amplitudes past any finite bound: as such sums end in FP32
-                    A[0].x = A[0].y = __int_as_float(0x7fffffff);
-                } else if (n_loud > 0) {
-                    add_loud(A, s.loud, n_loud, b);
-                }
+                if (any_bad && s.bad[b >> 5] >> (b & 31) & 1) A[0].x = A[0].y = __int_as_float(0x7fffffff);
 #pragma unroll
                 for (int p = 0; p < kMBasis; p++) {
                     // (high orders first: the small terms, so that fewer roundings are of full size)
@@ -949,7 +978,9 @@ void jacobi(Mat A, int n, Mat V) {
 // coefficients the basis vectors are found in three steps, each the leading eigenvectors of
 // a Gram matrix in what the steps before it leave: two for the taps beyond kMomFar samples,
 // one for those beyond kMomNear, the others for all taps (the last of those is not needed:
-// kMBasis).  Taps on which a pair's coefficients are below 2e-8 are left out of its runs.
+// kMBasis).  Taps count by their relative error down to 2 / H^2, so that the far taps of a lone
+// image are as good as its near ones (2e-7 of their size; unweighted the same 3e-8 of the whole,
+// but 2e-6 at 50 samples of a window of 128).  Taps on which a pair's coefficients are below 2e-8 are left out of its runs.
 // The vectors are orthonormal, so S and the coefficients are of order one; S is rounded to
 // FP32 first and the coefficients fitted to the rounded functions (with monomial moments
 // and plain rounding, the FP32 tables cost 2e-7).
@@ -999,6 +1030,7 @@ void moment_basis(int tw, MomBasis &B) {
     }
     std::vector<std::vector<double>> F(2 * J, std::vector<double>(n, 0.0));   // (even, odd) per pair
     const double beyond[3] = {kMomFar, kMomNear, -1.0};
+    const double quiet = 2.0 / (H * H);   // taps below this are weighted alike
     const int take[3] = {2, 1, kMPairs - 3};
     for (int par = 0; par < 2; par++) {
         Mat Q, rest;   // columns found so far; columns spanning what they leave
@@ -1009,13 +1041,15 @@ void moment_basis(int tw, MomBasis &B) {
             Mat G = {}, V, next;
             for (int m = 0; m < 2 * J; m++) {
                 if (std::fabs(kap[m]) <= beyond[step] || std::fabs(kap[m]) > H - 1.01) continue;   // (whole cells)
-                double y[kMPairs];
+                double y[kMPairs], size2 = 0.0;
+                for (int a = 0; a < kMPairs; a++) size2 += C[m][2 * a + par] * C[m][2 * a + par];
+                const double weight = 1.0 / (size2 + quiet * quiet);
                 for (int j = 0; j < nr; j++) {
                     y[j] = 0.0;
                     for (int a = 0; a < kMPairs; a++) y[j] += C[m][2 * a + par] * rest[a][j];
                 }
                 for (int i = 0; i < nr; i++)
-                    for (int j = 0; j < nr; j++) G[i][j] += y[i] * y[j];
+                    for (int j = 0; j < nr; j++) G[i][j] += weight * y[i] * y[j];
             }
             jacobi(G, nr, V);
             for (int a = 0; a < kMPairs; a++)
@@ -1164,7 +1198,7 @@ const MomBasis &moment_basis_cached(int tw) {
 int moment_cells(int T, const MomBasis &B) { return (T / 2 + 4 * B.quads + 8 + 7) / 8 * 8; }
 
 size_t moment_smem_bytes(int threads, int axis_cap, const MomBasis &B) {
-    size_t o[9];
+    size_t o[10];
     return threads == kMomSmall ? mom_layout<MomCfg<kMomSmall>>(B.n_quads, axis_cap, o)
                                 : mom_layout<MomCfg<kMomLarge>>(B.n_quads, axis_cap, o);
 }
