@@ -431,17 +431,20 @@ static int ensure_stage(gpurir_sim *s, size_t bytes) {
 }
 
 struct Plan {
-    int tpl, em, nsub, grid, clamp;
+    int tpl = 0, em = 0, nsub = 0, grid = 0, clamp = 0;
     long unfused_tails = 0;   // RIRs whose tail the separate tail kernel writes
     int axis_cap = 0;         // per-axis table entries per block (max over rooms of N0 + N1 + N2)
     std::vector<PartGroup> groups;   // partial segments to add up (RIRs split by images)
     long long part_floats = 0;       // size of the partial-segment buffer
     int max_part_len = 0;
     int mode = 0, tw = 0;   // tap evaluation mode (0 FP32, 1 mixed precision, 2 LUT), window length
-    int max_n_diff;
+    int max_n_diff = 0;
     bool skip_flags = false;   // some segment starts past the rooms' delay bound: test items on the device
-    // fractional-delay moment path (ism_moment.cu); nullptr: taps one by one (ism_forward.cu)
+    // rooms of the fractional-delay moment path (ism_moment.cu): the first n_mom items; the others'
+    // taps are summed one by one (ism_forward.cu)
     const MomBasis *mom = nullptr;
+    int n_mom = 0, mom_grid = 0, mom_axis_cap = 0;
+    long mom_rirs = 0;
     int mom_T = 0;                // longest segment
     int mom_win = 0;              // shortest last segment of an item
     int mom_threads = 0;          // shape of its blocks
@@ -483,9 +486,10 @@ static double room_span(const RoomDesc &r) {
 // what one block's shared memory holds; RIRs of small launches are cut finer so
 // that the persistent grid has work for every SM.  Items are ordered by an
 // estimate of their cost, largest first (longest-processing-time order).
-static int plan_taps(gpurir_sim *s, const std::vector<RoomDesc> &R, Plan &P) {
+// mom: rooms that are left to plan_moment (none if empty).
+static int plan_taps(gpurir_sim *s, const std::vector<RoomDesc> &R, Plan &P, const std::vector<char> &mom = {}) {
     int max_nsub = 0;
-    P.mom = nullptr;
+    auto theirs = [&](size_t ri) { return !mom.empty() && mom[ri]; };
     P.mode = s->lut ? 2 : (s->mp ? 1 : 0);
     if (P.mode != 0 && s->comp > 0) {   // compensated accumulation (mode flag 4, ism_forward.cu)
         int longest = 0;
@@ -496,21 +500,14 @@ static int plan_taps(gpurir_sim *s, const std::vector<RoomDesc> &R, Plan &P) {
     if (rc) return rc;
     const int sub = 32 * P.tpl;
     long M_tot = 0;
-    P.max_n_diff = 0;
-    P.axis_cap = 0;
-    for (const RoomDesc &r : R) {
+    for (size_t ri = 0; ri < R.size(); ri++) {
+        if (theirs(ri)) continue;
+        const RoomDesc &r = R[ri];
         M_tot += (long)r.n_src * r.n_rcv;
         P.max_n_diff = std::max(P.max_n_diff, r.n_total - r.n_ism);
         P.axis_cap = std::max(P.axis_cap, r.nb[0] + r.nb[1] + r.nb[2]);
     }
-    P.items.clear();
-    P.rirs.clear();
-    P.skip_flags = false;
-    P.groups.clear();
-    P.part_floats = 0;
-    P.max_part_len = 0;
-    P.unfused_tails = 0;
-    P.rirs.reserve(M_tot);
+    P.rirs.reserve(P.rirs.size() + M_tot);
     const long seg_max = std::min<long>((long)max_nsub * sub, 16384);   // int16 image offsets
     const long target = 4L * s->num_sms;
     const long want = (target + M_tot - 1) / std::max<long>(M_tot, 1);
@@ -520,6 +517,7 @@ static int plan_taps(gpurir_sim *s, const std::vector<RoomDesc> &R, Plan &P) {
     cost.reserve(M_tot);
     P.nsub = 1;
     for (size_t ri = 0; ri < R.size(); ri++) {
+        if (theirs(ri)) continue;
         const RoomDesc &r = R[ri];
         const long M = (long)r.n_src * r.n_rcv;
         long n_seg = 0, n_part = 1;
@@ -602,16 +600,15 @@ static int plan_taps(gpurir_sim *s, const std::vector<RoomDesc> &R, Plan &P) {
     if (!sorted)
         std::stable_sort(cost.begin(), cost.end(), [](const std::pair<double, int> &x,
                                                       const std::pair<double, int> &y) { return x.first > y.first; });
-    P.items.reserve(work.size());
+    P.items.reserve(P.items.size() + work.size());
     for (auto &c : cost) P.items.push_back(work[c.second]);
 
-    P.grid = 0;
-    if (P.items.empty()) return GPURIR_OK;
+    if (work.empty()) return GPURIR_OK;
     size_t smem = ism_forward_smem_bytes(P.tpl, P.em, P.nsub, P.mode, P.tw);
     int bps = ism_forward_blocks_per_sm(P.tpl, smem, P.mode);
     if (bps < 1) return fail(GPURIR_ERR_CUDA, "ISM kernel does not fit on an SM");
     if (tuning(1) > 0) bps = std::min(bps, tuning(1));   // ism_blocks_per_sm (tuning.cu)
-    P.grid = (int)std::min<long>((long)P.items.size(), (long)s->num_sms * bps);
+    P.grid = (int)std::min<long>((long)work.size(), (long)s->num_sms * bps);
     return GPURIR_OK;
 }
 
@@ -632,25 +629,17 @@ static double shell_images(const RoomDesc &r, double a, double b) {
 // long enough to hold its envelope window (so that its item writes the diffuse tail), and
 // in launches of few RIRs the image rows of heavy segments dealt to several items whose
 // partial segments are added up afterwards.
-static int plan_moment(gpurir_sim *s, const std::vector<RoomDesc> &R, Plan &P) {
+static int plan_moment(gpurir_sim *s, const std::vector<RoomDesc> &R, Plan &P, const std::vector<char> &mom) {
     P.mode = 0;
     P.tw = (int)std::lround(2.0 * R[0].H);
     P.mom = &moment_basis_cached(P.tw);
-    P.items.clear();
-    P.rirs.clear();
-    P.groups.clear();
-    P.skip_flags = false;
-    P.part_floats = 0;
-    P.max_part_len = 0;
-    P.unfused_tails = 0;
-    P.max_n_diff = 0;
-    P.axis_cap = 0;
-    long M_tot = 0;
     double covered = 0.0;   // samples of all early parts that an image can reach
-    for (const RoomDesc &r : R) {
-        M_tot += (long)r.n_src * r.n_rcv;
+    for (size_t ri = 0; ri < R.size(); ri++) {
+        if (!mom[ri]) continue;
+        const RoomDesc &r = R[ri];
+        P.mom_rirs += (long)r.n_src * r.n_rcv;
         P.max_n_diff = std::max(P.max_n_diff, r.n_total - r.n_ism);
-        P.axis_cap = std::max(P.axis_cap, r.nb[0] + r.nb[1] + r.nb[2]);
+        P.mom_axis_cap = std::max(P.mom_axis_cap, r.nb[0] + r.nb[1] + r.nb[2]);
         covered += (double)r.n_src * r.n_rcv * std::min<double>(r.n_ism, room_span(r));
     }
     // Costs in cycles of one SM with its blocks at work (measured, two large blocks): 2.8 per
@@ -666,6 +655,7 @@ static int plan_moment(gpurir_sim *s, const std::vector<RoomDesc> &R, Plan &P) {
         const double fixed = 0.14 * T * P.mom->n_quads + 3500.0;
         const int least = win <= T - 4 ? win : 0;
         for (size_t ri = 0; ri < R.size(); ri++) {
+            if (!mom[ri]) continue;
             const RoomDesc &r = R[ri];
             const double span = room_span(r);
             for (int a = 0, b; a < r.n_ism; a = b) {
@@ -723,8 +713,8 @@ static int plan_moment(gpurir_sim *s, const std::vector<RoomDesc> &R, Plan &P) {
             const float rest = threads == kMomSmall ? 0.8f : 1.0f;
             if (moment_cells(T, *P.mom) > (threads == kMomSmall ? kMomSmallCells : kMomCells)) continue;
             // (tables in global memory want the L1 that three blocks take: 48 rooms 278 us, with three 329)
-            if (threads == kMomSmall && (P.axis_cap > kMomTabSmem ||
-                                         moment_blocks_per_sm(threads, moment_smem_bytes(threads, P.axis_cap, *P.mom)) < 3)) continue;
+            if (threads == kMomSmall && (P.mom_axis_cap > kMomTabSmem ||
+                                         moment_blocks_per_sm(threads, moment_smem_bytes(threads, P.mom_axis_cap, *P.mom)) < 3)) continue;
             auto consider = [&](float limit) {
                 double n;
                 const double t = blocks * time_of(with, slots, rest, limit, n);
@@ -755,7 +745,7 @@ static int plan_moment(gpurir_sim *s, const std::vector<RoomDesc> &R, Plan &P) {
     if (segs.empty()) return fail(GPURIR_ERR_UNSUPPORTED, "window too long");   // (use_moments)
     const int T = P.mom_T;
     P.mom_win = win <= T - 4 ? win : 0;
-    P.mom_smem = moment_smem_bytes(P.mom_threads, P.axis_cap, *P.mom);
+    P.mom_smem = moment_smem_bytes(P.mom_threads, P.mom_axis_cap, *P.mom);
     int bps = moment_blocks_per_sm(P.mom_threads, P.mom_smem);
     if (bps < 1) return fail(GPURIR_ERR_CUDA, "ISM kernel does not fit on an SM");
     if (tuning(1) > 0) bps = std::min(bps, tuning(1));   // ism_blocks_per_sm (tuning.cu)
@@ -764,10 +754,11 @@ static int plan_moment(gpurir_sim *s, const std::vector<RoomDesc> &R, Plan &P) {
     for (const std::vector<Seg> &room : segs)
         for (const Seg &g : room) total += g.n * (g.images + g.rest);
     const double most = total / (4.0 * (P.mom_threads == kMomSmall ? 3.0 : 2.0) * s->num_sms);
-    P.rirs.reserve(M_tot);
+    P.rirs.reserve(P.mom_rirs);
     std::vector<IsmItem> work;
     std::vector<std::pair<double, int>> cost;
     for (size_t ri = 0; ri < R.size(); ri++) {
+        if (!mom[ri]) continue;
         const RoomDesc &r = R[ri];
         const long M = (long)r.n_src * r.n_rcv;
         // items of one RIR: a heavy segment as several interleaved parts, light ones in runs
@@ -826,16 +817,16 @@ static int plan_moment(gpurir_sim *s, const std::vector<RoomDesc> &R, Plan &P) {
     });
     P.items.reserve(work.size());
     for (auto &c : cost) P.items.push_back(work[c.second]);
-    P.grid = (int)std::min<long>((long)P.items.size(), (long)s->num_sms * bps);
+    P.n_mom = (int)P.items.size();
+    P.mom_grid = (int)std::min<long>((long)P.n_mom, (long)s->num_sms * bps);
     return GPURIR_OK;
 }
 
 // Which kernel evaluates a launch.  The moment kernel serves the default FP32 mode at window
 // lengths from 48 (6 kHz; below, the window's ends inside a cell cost accuracy) to 400
 // samples (50 kHz; its cells' sums and filter fill two blocks per SM there), when the RIRs
-// have images enough: a sample's filter costs what the taps of some tenths of an image do,
-// and an RIR of few images is nearer to the FP64 sum with the taps (a single image: 3e-8
-// against 9e-8).  The line is a mean of 2048 images in reach per RIR at a window of 128
+// have images enough: a sample's filter costs what the taps of some tenths of an image do.
+// The line is a mean of 2048 images in reach per RIR at a window of 128
 // samples, fewer for longer windows: measured over 150 launches of 1 to 800 RIRs, 1 to 400000
 // images each, 6 to 48 kHz, the moment kernel takes 0.21-0.5 of the tap kernel's time on dense
 // rooms, 0.5-0.8 at 3000 to 10000 images, 0.75-1.05 below 2000.
@@ -852,8 +843,25 @@ static bool use_moments(const gpurir_sim *s, const std::vector<RoomDesc> &R) {
     return images * tw >= 2048.0 * 128.0 * rirs;
 }
 
+// Rooms of a moment launch with fewer images in reach keep the taps, whatever the others are: an RIR
+// of few images is nearer to the FP64 sum with them (one image: 6.5e-8 against 1.1e-7; 8 images
+// 1.0e-7 and 1.2e-7; from 27 on the same).
+static const double kMomFewImages = 64.0;
+
 static int plan_rooms(gpurir_sim *s, const std::vector<RoomDesc> &R, Plan &P) {
-    return use_moments(s, R) ? plan_moment(s, R, P) : plan_taps(s, R, P);
+    P = Plan();
+    if (!use_moments(s, R)) return plan_taps(s, R, P);
+    std::vector<char> mom(R.size());
+    size_t n = 0;
+    for (size_t ri = 0; ri < R.size(); ri++) {
+        mom[ri] = shell_images(R[ri], 0.0, R[ri].n_ism + R[ri].H) >= kMomFewImages;
+        n += mom[ri];
+    }
+    int rc = plan_moment(s, R, P, mom);
+    if (rc || n == R.size()) return rc;
+    if ((rc = plan_taps(s, R, P, mom))) return rc;
+    std::sort(P.rirs.begin(), P.rirs.end(), [](const IsmItem &x, const IsmItem &y) { return x.rir < y.rir; });
+    return GPURIR_OK;
 }
 
 static int check_status(gpurir_sim *s) {
@@ -876,7 +884,7 @@ static Layout make_layout(const Plan &P, size_t n_rooms, long n_src, long n_rcv,
     Layout L;
     // rooms and positions first: the part of an upload that changes from call to call
     L.o_rooms = 0;
-    // work counter, zero in every upload: no memset per call (a plain room 82 to 74 us)
+    // work counters of both kernels, zero in every upload: no memset per call (a plain room 82 to 74 us)
     L.o_work = align_up(n_rooms * sizeof(RoomDesc), 16);
     L.o_pos = align_up(L.o_work + 16, 256);
     size_t n_pos = host_io ? (size_t)(n_src + n_rcv) * 3 * 2 : 0;
@@ -888,8 +896,8 @@ static Layout make_layout(const Plan &P, size_t n_rooms, long n_src, long n_rcv,
     L.stage_bytes = align_up(L.o_coef + (P.mom ? P.mom->coef.size() * sizeof(float2) : 0), 256);
     L.o_env = L.stage_bytes;
     L.o_axis = align_up(L.o_env + (size_t)M * 3 * sizeof(float), 256);
-    // (the moment kernel holds the tables of two items per block)
-    L.o_part = align_up(L.o_axis + (size_t)P.grid * P.axis_cap * (P.mom ? 2 : 1) * sizeof(float4), 256);
+    // (one kernel's after the other's; the moment kernel holds the tables of two items per block)
+    L.o_part = align_up(L.o_axis + std::max((size_t)P.grid * P.axis_cap, (size_t)P.mom_grid * P.mom_axis_cap * 2) * sizeof(float4), 256);
     L.o_skip = align_up(L.o_part + (size_t)P.part_floats * sizeof(float), 256);
     L.o_out = align_up(L.o_skip + (P.skip_flags ? P.items.size() : 0), 256);
     L.dev_bytes = L.o_out + (host_io ? (size_t)out_elems * sizeof(float) : 0);
@@ -953,7 +961,8 @@ static int enqueue_kernels(gpurir_sim *s, const Plan &P, const char *d, const La
                            cudaStream_t st, bool record, bool skip_ready = false,
                            const unsigned char *tail_pre = nullptr) {
     const RoomDesc *drooms = reinterpret_cast<const RoomDesc *>(d + L.o_rooms);
-    if (record && s->profile && P.grid > 0) { CK(cudaEventRecord(s->ev[0], st)); s->ev_ism = true; }
+    const bool any = P.grid + P.mom_grid > 0;
+    if (record && s->profile && any) { CK(cudaEventRecord(s->ev[0], st)); s->ev_ism = true; }
     TailArgs ta;
     ta.seed = s->seed;
     ta.offset = s->calls;
@@ -963,30 +972,31 @@ static int enqueue_kernels(gpurir_sim *s, const Plan &P, const char *d, const La
     ta.fuse = 1;
     ta.pre = tail_pre;
     if (record) {
-        s->last_launches = (P.grid > 0 ? 1 : 0);
-        s->last_moment_rirs = P.mom && P.grid > 0 ? M : 0;
+        s->last_launches = (P.grid > 0) + (P.mom_grid > 0);
+        s->last_moment_rirs = P.mom_grid > 0 ? P.mom_rirs : 0;
     }
+    const IsmItem *items = reinterpret_cast<const IsmItem *>(d + L.o_items), *tap_items = items + P.n_mom;
+    const int n_tap_items = (int)P.items.size() - P.n_mom;
     unsigned char *skip = nullptr;
     if (P.grid > 0 && P.skip_flags) {   // segments no image may reach: flags at the current positions
         skip = reinterpret_cast<unsigned char *>(const_cast<char *>(d) + L.o_skip);
         if (!skip_ready) {   // (else written by room_beta_skip_kernel just before)
-            CK(item_skip_launch(drooms, reinterpret_cast<const IsmItem *>(d + L.o_items), (int)P.items.size(),
-                                dps, dpr, skip, st));
+            CK(item_skip_launch(drooms, tap_items, n_tap_items, dps, dpr, skip, st));
             if (record) s->last_launches += 1;
         }
     }
-    if (P.grid > 0 && P.mom) {
+    if (P.mom_grid > 0) {
         MomLaunch m{};
         m.rooms = drooms;
-        m.items = reinterpret_cast<const IsmItem *>(d + L.o_items);
-        m.n_items = (int)P.items.size();
+        m.items = items;
+        m.n_items = P.n_mom;
         m.pos_src = dps; m.pos_rcv = dpr; m.orv_src = dos; m.orv_rcv = dor;
         m.out = dout;
         m.partial = reinterpret_cast<float *>(const_cast<char *>(d) + L.o_part);
-        m.work_counter = work_counter;
+        m.work_counter = work_counter + 1;
         m.status = s->h_ctl + 1;
         m.axis_tab = reinterpret_cast<float4 *>(const_cast<char *>(d) + L.o_axis);
-        m.axis_cap = P.axis_cap;
+        m.axis_cap = P.mom_axis_cap;
         m.T = P.mom_T;
         m.win = P.mom_win;
         m.lead = P.mom->lead;
@@ -999,10 +1009,10 @@ static int enqueue_kernels(gpurir_sim *s, const Plan &P, const char *d, const La
         memcpy(m.S, P.mom->S, sizeof(m.S));
         m.seed = ta.seed; m.offset = ta.offset; m.offset_ptr = ta.offset_ptr;
         m.noise_kind = ta.noise_kind; m.env_out = ta.env_out; m.fuse_tail = ta.fuse; m.tail_pre = ta.pre;
-        CK(moment_launch(m, P.mom_threads, P.mom_smem, P.grid, st));
-    } else if (P.grid > 0)
-        CK(ism_forward_launch(P.tpl, drooms, reinterpret_cast<const IsmItem *>(d + L.o_items),
-                              (int)P.items.size(), dps, dpr, dos, dor, dout, work_counter,
+        CK(moment_launch(m, P.mom_threads, P.mom_smem, P.mom_grid, st));
+    }
+    if (P.grid > 0)
+        CK(ism_forward_launch(P.tpl, drooms, tap_items, n_tap_items, dps, dpr, dos, dor, dout, work_counter,
                               s->h_ctl + 1, P.em, P.nsub, P.clamp, P.grid, st, P.mode, P.tw, &ta,
                               reinterpret_cast<float4 *>(const_cast<char *>(d) + L.o_axis), P.axis_cap,
                               reinterpret_cast<float *>(const_cast<char *>(d) + L.o_part), skip));
@@ -1012,7 +1022,7 @@ static int enqueue_kernels(gpurir_sim *s, const Plan &P, const char *d, const La
                                  P.max_part_len, reinterpret_cast<const float *>(d + L.o_part), dout, st));
     }
     if (record && s->ev_ism) CK(cudaEventRecord(s->ev[1], st));
-    const bool tail_kernel = P.max_n_diff > 0 && (P.unfused_tails > 0 || P.grid == 0);
+    const bool tail_kernel = P.max_n_diff > 0 && (P.unfused_tails > 0 || !any);
     if (record && s->profile && tail_kernel) { CK(cudaEventRecord(s->ev[2], st)); s->ev_tail = true; }
     if (record && tail_kernel) s->last_launches += 1;
     if (tail_kernel)
@@ -1193,7 +1203,7 @@ static int simulate_rooms(gpurir_sim *s, std::vector<RoomDesc> &R, long n_src, l
     // ... and, into page-locked memory, tails silent by geometry are streamed by a copy
     // engine meanwhile
     bool pre = false;
-    if (host_io && pinned && P.grid > 0 && P.max_n_diff > 0)
+    if (host_io && pinned && P.grid + P.mom_grid > 0 && P.max_n_diff > 0)
         if ((rc = stream_silent_tails(s, R, P, pos_src, pos_rcv, out,
                                       reinterpret_cast<unsigned char *>(h + L.o_pre), pre)))
             return rc;
@@ -1434,7 +1444,7 @@ static int batch_device(gpurir_sim *s, int n_rooms, const gpurir_room *rooms, fl
 // ---------------------------------------------------------------------------
 struct gpurir_batch {
     gpurir_sim *sim = nullptr;
-    char *d = nullptr;            // descriptors + envelope + work counter + call offset
+    char *d = nullptr;            // descriptors + envelope + work counters + call offset
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     long n_rir = 0;
@@ -1461,7 +1471,7 @@ extern "C" int gpurir_batch_create(gpurir_sim *s, int n_rooms, const gpurir_room
     if ((rc = plan_rooms(s, R, P))) return rc;
     const long M = (long)P.rirs.size();
     Layout L = make_layout(P, R.size(), ns, nr, M, tot, false);
-    const size_t o_ctl = align_up(L.o_out, 256);           // work counter, then the call offset
+    const size_t o_ctl = align_up(L.o_out, 256);           // two work counters, then the call offset
     const size_t bytes = o_ctl + 256;
     std::vector<char> h(L.stage_bytes);
     fill_stage(h.data(), L, R, P);
@@ -1484,7 +1494,7 @@ extern "C" int gpurir_batch_create(gpurir_sim *s, int n_rooms, const gpurir_room
     uint64_t *offset = reinterpret_cast<uint64_t *>(b->d + o_ctl + 8);
     e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
-        cudaMemsetAsync(counter, 0, sizeof(int), cap);   // (a failure shows at the end of the capture)
+        cudaMemsetAsync(counter, 0, 2 * sizeof(int), cap);   // (a failure shows at the end of the capture)
         rc = enqueue_kernels(s, P, b->d, L, M, d_pos_src, d_pos_rcv, d_orV_src, d_orV_rcv, d_out,
                              counter, offset, cap, false);
         if (rc == GPURIR_OK && P.max_n_diff > 0) {
