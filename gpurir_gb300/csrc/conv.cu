@@ -1388,6 +1388,9 @@ cudaError_t traj_adjoint_launch(const double *g, long n_out, const int *w_ini, c
 __global__ void ola_kernel(const float *conv, long conv_ld, const int *w_ini, const int *w_len, int P,
                            int R, int L, long n_out, int uni_w, double *out) {
     after_previous();
+    conv = after_wait(conv);
+    w_ini = after_wait(w_ini);
+    w_len = after_wait(w_len);
     const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;   // consecutive t: coalesced reads
     const int r = blockIdx.y;
     if (t >= n_out) return;
