@@ -401,12 +401,17 @@ __device__ __forceinline__ void reg_fft(float2 (&v)[16], float2 *buf, const floa
 // block copies them once; read from the table in global memory, whose stride of
 // 2M / 16 Ns elements spreads a warp over up to 32 lines, they were 40 % of the load
 // pipe's wavefronts and the longest stall (8192 points, 3200 rows: 244 us, with the tables 215).
-template <int M>
+// One row per block leaves the spectral step's factors in global memory, where consecutive
+// threads read consecutive ones: with them a second block would not fit on the SM.
+template <int M, int ROWS>
 struct RowTw {
     static constexpr bool fused = M == 8192;               // radix-2 passes folded into the spectral step
     static constexpr int head = 4 * 16 + (M >= 4096 ? 4 * 256 : 0);
     static constexpr int tail = fused ? 4 * (2 + 32 + 512) : 0;
-    static constexpr int bins = fused ? M / 2 : 0;         // W[u], then W[2u], u < M/4: the spectral step's
+    static constexpr int bins = fused && ROWS > 1 ? M / 2 : 0;   // W[u], then W[2u], u < M/4: the spectral step's
+    static constexpr int blocks = 16384 / M / ROWS > 0 ? 16384 / M / ROWS : 1;   // per SM
+    static constexpr size_t smem = ((size_t)ROWS * (M + M / 16) + head + tail + bins) * sizeof(float2);
+    static_assert(blocks * (smem + 1024) <= 228 * 1024, "resident blocks fit the SM's shared memory");
 };
 template <int M>
 __device__ __forceinline__ void row_twiddles_pass(float2 *tw, int Ns, const float2 *__restrict__ W) {
@@ -415,16 +420,16 @@ __device__ __forceinline__ void row_twiddles_pass(float2 *tw, int Ns, const floa
         tw[e] = __ldg(&W[(k << i) * ((2 * M) / (Ns * 16))]);
     }
 }
-template <int M>
+template <int M, int ROWS>
 __device__ __forceinline__ void row_twiddles(float2 *tw, const float2 *__restrict__ W) {
     row_twiddles_pass<M>(tw, 16, W);
     if (M >= 4096) row_twiddles_pass<M>(tw + 64, 256, W);
-    if (RowTw<M>::fused) {
-        row_twiddles_pass<M>(tw + RowTw<M>::head, 2, W);
-        row_twiddles_pass<M>(tw + RowTw<M>::head + 8, 32, W);
-        row_twiddles_pass<M>(tw + RowTw<M>::head + 136, 512, W);
-        float2 *b = tw + RowTw<M>::head + RowTw<M>::tail;
-        for (int u = threadIdx.x; u < M / 4; u += M / 16) {
+    if (RowTw<M, ROWS>::fused) {
+        row_twiddles_pass<M>(tw + RowTw<M, ROWS>::head, 2, W);
+        row_twiddles_pass<M>(tw + RowTw<M, ROWS>::head + 8, 32, W);
+        row_twiddles_pass<M>(tw + RowTw<M, ROWS>::head + 136, 512, W);
+        float2 *b = tw + RowTw<M, ROWS>::head + RowTw<M, ROWS>::tail;
+        for (int u = threadIdx.x; u < RowTw<M, ROWS>::bins / 2; u += M / 16) {
             b[u] = __ldg(&W[u]);
             b[M / 4 + u] = __ldg(&W[2 * u]);
         }
@@ -657,10 +662,12 @@ __device__ __forceinline__ void conv_spectral_fused(float2 (&v)[ROWS][16], float
     constexpr int T = M / 16, BS = M + M / 16, H = M / 2, Q = M / 4;
     static_assert(Q == 4 * T, "four units per thread");
     const int j = threadIdx.x;
-    const float2 *wb = tw + RowTw<M>::head + RowTw<M>::tail;
+    const float2 *wb = tw + RowTw<M, ROWS>::head + RowTw<M, ROWS>::tail;
+    auto w1 = [&](int u) { return RowTw<M, ROWS>::bins > 0 ? wb[u] : __ldg(&W[u]); };            // W[u], u < M/4
+    auto w2 = [&](int u) { return RowTw<M, ROWS>::bins > 0 ? wb[Q + u] : __ldg(&W[2 * u]); };    // W[2u]
     reg_fft_rows_head<false, M, ROWS>(v, buf, tw);
     // segment spectrum at the thread's bins k, M - k, k', M - k' (rows of one point share it):
-    // asked for before the barrier
+    // asked for before the barrier, where registers allow it (one row per block has 64 a thread)
     float2 s4[4][4];
     const int p0 = pr0 / R;
     auto spectrum = [&](int p) {
@@ -674,7 +681,7 @@ __device__ __forceinline__ void conv_spectral_fused(float2 (&v)[ROWS][16], float
             s4[i][3] = __ldg(&sp[M - kp]);
         }
     };
-    spectrum(p0);
+    if (ROWS > 1) spectrum(p0);
     float2 e[ROWS][2];   // unit M/4 (thread 0 only): Z[M/4], Z[3M/4]
 #pragma unroll
     for (int q = 0; q < ROWS; q++) {
@@ -683,12 +690,12 @@ __device__ __forceinline__ void conv_spectral_fused(float2 (&v)[ROWS][16], float
         for (int i = 0; i < 4; i++) {
             const int u = j + i * T;
             if (u == 0) {   // bins 0 and M/2: Z[0] = A[0] + B[0], Z[M/2] = A[0] - B[0]
-                float2 a0 = bq[pad16(0)], a1 = cmul(bq[pad16(H)], wb[0]);
+                float2 a0 = bq[pad16(0)], a1 = cmul(bq[pad16(H)], w1(0));
                 v[q][4 * i] = cadd(a0, a1);
                 v[q][4 * i + 1] = csub(a0, a1);
             } else {
                 const int k = u, kp = H - u;
-                const float2 w = wb[Q + u], wp = make_float2(-w.x, w.y);   // W[2k], W[2k']
+                const float2 w = w2(u), wp = make_float2(-w.x, w.y);   // W[2k], W[2k']
                 const float2 ak = bq[pad16(k)], bk = cmul(bq[pad16(k + H)], w);
                 const float2 ap = bq[pad16(kp)], bp = cmul(bq[pad16(kp + H)], wp);
                 v[q][4 * i] = cadd(ak, bk);        // Z[k]
@@ -710,13 +717,13 @@ __device__ __forceinline__ void conv_spectral_fused(float2 (&v)[ROWS][16], float
         float2 *bq = buf + q * BS;
         const int p = (pr0 + q) / R;
         const float2 *sp = Sg + (size_t)p * (M + 1);
-        if (q > 0 && p != (pr0 + q - 1) / R) spectrum(p);
+        if (ROWS == 1 || (q > 0 && p != (pr0 + q - 1) / R)) spectrum(p);
 #pragma unroll
         for (int i = 0; i < 4; i++) {
             const int u = j + i * T;
             if (u == 0) {
                 float2 y0, yM, yh, yh2;
-                conv_bin_pair(v[q][0], v[q][0], wb[0], s4[i][0], s4[i][1], y0, yM);
+                conv_bin_pair(v[q][0], v[q][0], w1(0), s4[i][0], s4[i][1], y0, yM);
                 conv_bin_pair(v[q][1], v[q][1], __ldg(&W[H]), s4[i][2], s4[i][3], yh, yh2);
                 bq[pad16(0)] = cadd(y0, yh);
                 bq[pad16(1)] = csub(y0, yh);
@@ -724,7 +731,7 @@ __device__ __forceinline__ void conv_spectral_fused(float2 (&v)[ROWS][16], float
                 const int k = u, kp = H - u;
                 float2 yk, ymk, ykp, ymkp;
                 // pair (k, M - k): Z[k], Z[M - k] = Z[k' + M/2]; pair (k', M - k'): Z[k'], Z[k + M/2]
-                const float2 w = wb[u], wp = make_float2(-w.y, -w.x);   // W[k], W[k']
+                const float2 w = w1(u), wp = make_float2(-w.y, -w.x);   // W[k], W[k']
                 conv_bin_pair(v[q][4 * i], v[q][4 * i + 3], w, s4[i][0], s4[i][1], yk, ymk);
                 conv_bin_pair(v[q][4 * i + 2], v[q][4 * i + 1], wp, s4[i][2], s4[i][3], ykp, ymkp);
                 // the inverse's first radix-2 pass: out[2j] = Y'[j] + Y'[j + M/2], out[2j + 1] = difference
@@ -742,11 +749,11 @@ __device__ __forceinline__ void conv_spectral_fused(float2 (&v)[ROWS][16], float
         }
     }
     __syncthreads();
-    reg_fft_rows_tail<true, M, ROWS>(v, buf, tw + RowTw<M>::head);
+    reg_fft_rows_tail<true, M, ROWS>(v, buf, tw + RowTw<M, ROWS>::head);
 }
 
 template <int M, int ROWS>
-__global__ void __launch_bounds__(M / 16, (16384 / M / ROWS > 0 ? 16384 / M / ROWS : 1)) rir_conv_reg_kernel(
+__global__ void __launch_bounds__(M / 16, (RowTw<M, ROWS>::blocks)) rir_conv_reg_kernel(
         const float *__restrict__ rir, int P, int R, int L, int S, const float2 *__restrict__ W,
         const float2 *__restrict__ Sg, float *__restrict__ out, long out_ld) {
     after_previous();
@@ -757,7 +764,7 @@ __global__ void __launch_bounds__(M / 16, (16384 / M / ROWS > 0 ? 16384 / M / RO
     extern __shared__ __align__(16) float2 sm[];
     float2 *buf = sm;   // ROWS buffers of pad16(M) elements
     float2 *tw = sm + ROWS * BS;
-    row_twiddles<M>(tw, W);   // (the first pass needs none: its barrier is before their first use)
+    row_twiddles<M, ROWS>(tw, W);   // (the first pass needs none: its barrier is before their first use)
     const int j = threadIdx.x;
     const int n_out = S + L - 1;
     float2 v[ROWS][16];
@@ -859,7 +866,7 @@ constexpr int kTuneTrajBlocksKnob = 3; // TuneKnob::kTuneTrajBlocksPerSm
 template <int M, int ROWS>
 static cudaError_t launch_reg_conv_rows(const float *rir, int P, int R, int L, int S, const float2 *W,
                                         const float2 *Sg, float *out, long out_ld, cudaStream_t st) {
-    const size_t smem = ((size_t)ROWS * (M + M / 16) + RowTw<M>::head + RowTw<M>::tail + RowTw<M>::bins) * sizeof(float2);
+    constexpr size_t smem = RowTw<M, ROWS>::smem;
     static int blocks = -1;
     if (blocks < 0) {
         cudaError_t e = cudaFuncSetAttribute(rir_conv_reg_kernel<M, ROWS>,
@@ -876,8 +883,10 @@ static cudaError_t launch_reg_conv_rows(const float *rir, int P, int R, int L, i
     return launch_after(rir_conv_reg_kernel<M, ROWS>, grid, M / 16, smem, st, rir, P, R, L, S, W, Sg, out, out_ld);
 }
 
-// Rows per block from the tuning table (1: more blocks per SM; 2: twiddles and
+// Rows per block from the tuning table (1: twice the blocks per SM; 2: twiddles and
 // barriers shared by a pair of rows).  Each row's arithmetic is the same either way.
+// (3200 rows of 8192 points: 265 us with one row, 249 with two, spectra of the segments and cold
+// inputs included; with all twiddles in shared memory one row had one block per SM and took 283.)
 template <int M>
 static cudaError_t launch_reg_conv(const float *rir, int P, int R, int L, int S, const float2 *W,
                                    const float2 *Sg, float *out, long out_ld, cudaStream_t st) {
