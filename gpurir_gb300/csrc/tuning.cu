@@ -30,7 +30,7 @@ static const KnobInfo kKnobs[kTuneCount] = {
     {"conv_rows", 2, 1, 2},               // RIR rows transformed together per block (convolution)
     {"ism_blocks_per_sm", 0, 0, 4},       // forward ISM kernel: 0 = as many as fit
     {"adjoint_blocks_per_sm", 0, 0, 8},   // adjoint ISM kernel: 0 = as many as fit
-    {"traj_adjoint_blocks_per_sm", 0, 0, 2},  // trajectory adjoint: 0 = 1 at N = 16384, else 2
+    {"traj_adjoint_blocks_per_sm", 0, 0, 2},  // trajectory adjoint by whole rows: 0 = 1 at N = 16384, else 2
 };
 
 static std::atomic<int> g_knob[kTuneCount] = {{2}, {0}, {0}, {0}};

@@ -189,20 +189,27 @@ def _case_adjoint(sim, dev):
     return run
 
 
+# Points, receivers, RIR and segment length of the case of traj_adjoint_blocks_per_sm: segments too
+# long for the adjoint in blocks of lags, which has no such choice (400 samples there: 0.277 ms at
+# any value of the knob).
+TRAJ_ADJOINT = (400, 8, 12800, 1200)
+
+
 def _case_traj_adjoint(sim, dev):
     import torch
+    P, R, N, S = TRAJ_ADJOINT
     g = torch.Generator(device=dev).manual_seed(5)
-    rir = torch.randn((400, 8, 12800), device=dev, generator=g) * 0.01
-    seg = torch.randn((400, 400), device=dev, generator=g)
-    gout = torch.randn((160000 + 12799, 8), device=dev, dtype=torch.float64, generator=g)
-    gs = torch.empty(160000, device=dev)
+    rir = torch.randn((P, R, N), device=dev, generator=g) * 0.01
+    seg = torch.randn((P, S), device=dev, generator=g)
+    gout = torch.randn((P * S + N - 1, R), device=dev, dtype=torch.float64, generator=g)
+    gs = torch.empty(P * S, device=dev)
     gr = torch.empty_like(rir)
-    w = np.ascontiguousarray((np.arange(401) * 400).astype(np.int32))
+    w = np.ascontiguousarray((np.arange(P + 1) * S).astype(np.int32))
     L = _lib.load()
 
     def run():
         _lib.check(L.gpurir_trajectory_adjoint_device(
-            sim.handle, seg.data_ptr(), 400, 400, w.ctypes.data_as(_lib.iptr), rir.data_ptr(), 8, 12800,
+            sim.handle, seg.data_ptr(), P, S, w.ctypes.data_as(_lib.iptr), rir.data_ptr(), R, N,
             gout.data_ptr(), gs.data_ptr(), gr.data_ptr(), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)),
             "gpurir_trajectory_adjoint_device")
         return torch.cat([gs, gr.ravel()])
