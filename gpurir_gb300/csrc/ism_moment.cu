@@ -47,8 +47,8 @@
 // cells, 3.6 wavefronts; an FP32 atomicAdd takes 9.3 cycles) where images are many -- the
 // load pipe is at 77 % on 128 rooms -- and issue with the phases' barriers where they are few
 // (56 % of the slots on the array).  Per launch, ism_forward.cu and this kernel: one dense RIR of
-// 6 million images 531 and 95 us, 64 x 32 array 490 and 322, 128 rooms 2680 and 670, 15 RIRs at
-// 48 kHz 87 and 37 (with one scale per segment 90, 321, 625 and 37).  (Other ways that were built first: a counting sort by cell with one
+// 6 million images 531 and 95 us, 64 x 32 array 490 and 322, 128 rooms 2680 and 645, 15 RIRs at
+// 48 kHz 87 and 37 (with one scale per segment 90, 321, 617 and 37).  (Other ways that were built first: a counting sort by cell with one
 // thread per cell adding in image order needed 8 barriers per 1024 images and ran at 228
 // cycles per 32 images and SM, against 90 here.)
 #include <algorithm>
@@ -305,7 +305,7 @@ __device__ __forceinline__ void ctx_finish(MomCtx &c, const MomLaunch &P, int id
     }
     v2 = __shfl_sync(0xffffffffu, v2, 0) + __shfl_sync(0xffffffffu, v2, 1) + __shfl_sync(0xffffffffu, v2, 2);
     if (lane == 0) {
-        // (a NaN or a huge bound: no image is ruled out)
+        // (a huge bound: no image is ruled out; of a position that is not a number no delay is one)
         const float far = sqrtf(v2) * (R.kh + R.kl) * 1.00001f + 4.0f;
         c.reach = far < 1.0e9f ? (int)far : 0x3fffffff;
         c.inv_k = 1.0f / R.kh;
@@ -512,10 +512,11 @@ __global__ void __launch_bounds__(THREADS, MomCfg<THREADS>::blocks) ism_moment_k
                 // image at least d_lo away one component is d_lo / sqrt(3) at least, which bounds its attenuation
                 // (walls that amplify too), and amplitudes are at most that bound over 4 pi d with d the shell's
                 // inner radius or the nearest image's distance.  An image's error of 2e-10 of that bound is then at
-                // most 3e-8 of the quiet ones.  Else every eight cells (16 samples) have a scale of their own, from
+                // most 5e-8 of the quiet ones.  Else every eight cells (16 samples) have a scale of their own, from
                 // the loudest of their images.  (With one scale always, 128 samples of a first segment were off by
                 // 2e-4 at 16 kHz and 0.15 at 8 kHz with walls of 0.1, by 2e-6 and 1.5e-4 with walls of 0.3; now 4e-7
-                // at most.  With a scale per eight cells always, 128 rooms take 887 us instead of 670.)
+                // at most.  With a scale per eight cells always, 128 rooms take 887 us; with the line at 128, 673 us
+                // and the same errors; here 645.)
                 int uniform = 0;
                 bool quiet = false;
                 if (span == 0) {
@@ -526,8 +527,8 @@ __global__ void __launch_bounds__(THREADS, MomCfg<THREADS>::blocks) ism_moment_k
                                               __int_as_float(C.near2[2])) * 0.999f;
                     const float near = fmaxf(d_lo, first), peak = att_max * 1.001f / near;
                     quiet = max(max(ctl[4], ctl[5]), ctl[6]) >= 0x7f800000 ||   // (a factor that is not finite)
-                            !(peak < 3.0e38f && peak * near <= 128.0f * __int_as_float(ctl[10]) &&
-                              peak * d_hi <= 128.0f * __int_as_float(ctl[11]));
+                            !(peak < 3.0e38f && peak * near <= 256.0f * __int_as_float(ctl[10]) &&
+                              peak * d_hi <= 256.0f * __int_as_float(ctl[11]));
                     uniform = __float_as_int(peak);
                 }
                 int placed = 0;
