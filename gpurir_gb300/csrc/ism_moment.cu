@@ -47,7 +47,7 @@
 // cells, 3.6 wavefronts; an FP32 atomicAdd takes 9.3 cycles) where images are many -- the
 // load pipe is at 77 % on 128 rooms -- and issue with the phases' barriers where they are few
 // (56 % of the slots on the array).  Per launch, ism_forward.cu and this kernel: one dense RIR of
-// 6 million images 531 and 95 us, 64 x 32 array 490 and 322, 128 rooms 2680 and 645, 15 RIRs at
+// 6 million images 531 and 92 us, 64 x 32 array 490 and 321, 128 rooms 2680 and 642, 15 RIRs at
 // 48 kHz 87 and 37 (with one scale per segment 90, 321, 617 and 37).  (Other ways that were built first: a counting sort by cell with one
 // thread per cell adding in image order needed 8 barriers per 1024 images and ran at 228
 // cycles per 32 images and SM, against 90 here.)
@@ -359,6 +359,13 @@ __device__ __forceinline__ void image_moments(float a, float u, Put put) {
     }
 }
 
+// Scale (its bits) of cells whose images have at most this peak / 4 pi (bits): 2^(e + 1) bounds them, with
+// room for the peak's rounding, and the steps' span covers that.
+__device__ __forceinline__ int scale_of(int peak, int span) {
+    const int e = (__float_as_int(__int_as_float(peak) * 0.0797f) >> 23) - 127;
+    return (127 + min(max(span - 1 - e, -120), 120)) << 23;
+}
+
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS, MomCfg<THREADS>::blocks) ism_moment_kernel(const __grid_constant__ MomLaunch P) {
     using Cfg = MomCfg<THREADS>;
@@ -460,7 +467,7 @@ __global__ void __launch_bounds__(THREADS, MomCfg<THREADS>::blocks) ism_moment_k
             while (bits < kMPMaxBits && 4.0f * mean + 24.0f > (float)(7 << bits >> 3)) bits++;
             bool packed = 2.0f * mean + 24.0f <= (float)(7 << bits >> 3);
             int shift = 0;     // bits given up to hold more images per cell
-            int span = 0;      // log2 of the steps that cover an amplitude, of the scales at hand
+            int span = 0;      // log2 of the steps that cover an amplitude
             int n_rows = 0, n_img = 0;
             bool rows_ready = false;   // a segment's only batch of rows stays in place
             for (;;) {
@@ -469,10 +476,11 @@ __global__ void __launch_bounds__(THREADS, MomCfg<THREADS>::blocks) ism_moment_k
                     for (int i = lane; 4 * i < nbe; i += 32)
                         reinterpret_cast<int4 *>(s.sum + a * kMStride)[i] = make_int4(0, 0, 0, 0);
                 if (tid < 4) ctl[tid] = tid == 1 ? -1 : 0;
-                const int spans = packed ? kMPSpan : 20 - shift;
-                const float most = __int_as_float((127 + spans) << 23);
+                const int before = span;
+                span = packed ? kMPSpan : 20 - shift;
+                const float most = __int_as_float((127 + span) << 23);
                 const float fine = packed ? __int_as_float((127 + 16 - bits) << 23) : most;   // steps of the second integer in one of the first
-                if (span == 0) {
+                if (before == 0) {
                     if (tid < kMScales) s.scale[tid] = 0;
                     else if (tid - kMScales < kMomCells / 32) s.bad[tid - kMScales] = 0;
                     if (warp < 3) {   // largest |attenuation| along one axis, and beyond d_lo / sqrt(3)
@@ -516,10 +524,9 @@ __global__ void __launch_bounds__(THREADS, MomCfg<THREADS>::blocks) ism_moment_k
                 // the loudest of their images.  (With one scale always, 128 samples of a first segment were off by
                 // 2e-4 at 16 kHz and 0.15 at 8 kHz with walls of 0.1, by 2e-6 and 1.5e-4 with walls of 0.3; now 4e-7
                 // at most.  With a scale per eight cells always, 128 rooms take 887 us; with the line at 128, 673 us
-                // and the same errors; here 645.)
-                int uniform = 0;
+                // and the same errors; here 642.)
                 bool quiet = false;
-                if (span == 0) {
+                if (before == 0) {
                     const float f0 = __int_as_float(ctl[4]), f1 = __int_as_float(ctl[5]), f2 = __int_as_float(ctl[6]);
                     const float att_max = fmaxf(fmaxf(__int_as_float(ctl[7]) * (f1 * f2), __int_as_float(ctl[8]) * (f0 * f2)),
                                                 __int_as_float(ctl[9]) * (f0 * f1));
@@ -529,21 +536,19 @@ __global__ void __launch_bounds__(THREADS, MomCfg<THREADS>::blocks) ism_moment_k
                     quiet = max(max(ctl[4], ctl[5]), ctl[6]) >= 0x7f800000 ||   // (a factor that is not finite)
                             !(peak < 3.0e38f && peak * near <= 256.0f * __int_as_float(ctl[10]) &&
                               peak * d_hi <= 256.0f * __int_as_float(ctl[11]));
-                    uniform = __float_as_int(peak);
+                    if (!quiet && tid < kMScales) s.scale[tid] = scale_of(__float_as_int(peak), span);
+                } else if (tid < kMScales) {
+                    s.scale[tid] += (span - before) * (1 << 23);
                 }
                 int placed = 0;
                 // twice over the images of a quiet segment: the loudest of every eight cells, by an estimate of
                 // distance and amplitude that is good to 1e-6; then the sums, at the scales that follow
                 for (int sums = !quiet; sums < 2; sums++) {
                 if (sums) {
-                    if (quiet) __syncthreads();   // peaks complete
-                    if (tid < kMScales) {   // 2^(e + 1) bounds the amplitudes of these eight cells; the steps' span covers that
-                        const int v = span > 0 || quiet ? s.scale[tid] : uniform;
-                        const int e = (__float_as_int(__int_as_float(v) * 0.0797f) >> 23) - 127;   // (1 / 4 pi, and room for rounding)
-                        s.scale[tid] = span == 0 ? (127 + min(max(spans - 1 - e, -120), 120)) << 23
-                                                 : v + (spans - span) * (1 << 23);
+                    if (quiet) {
+                        __syncthreads();   // peaks complete
+                        if (tid < kMScales) s.scale[tid] = scale_of(s.scale[tid], span);
                     }
-                    span = spans;
                     if (rows_ready) __syncthreads();   // (else the rows' barriers come first)
                 }
                 for (int rbase = 0; rbase < my_rows; rbase += batch) {
