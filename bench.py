@@ -37,8 +37,11 @@ METRIC = ("RIRs/s & image-sample updates/s, batched vs plain fwd; fwd+adjoint st
 WORKLOAD = "mic_array"
 WORKLOAD_DESC = ("mic_array: room 6x5x3 m, Sabine beta (T60 1.0 s), 64 omni src x 32 cardioid rcv, "
                  "nb_img [12,14,24], Tdiff 0.3 s, Tmax 1.0 s, fs 16 kHz, Gaussian tail, FP32")
-FLOPS_PER_UPDATE = 8      # FP32 ops per windowed update of the reference formula
-SFU_PER_UPDATE = 3        # transcendental ops (sin, cos, reciprocal) per update
+# FP32 operations of the moment kernel at 16 kHz (a multiply-add counts two): per image its
+# float-float delay and amplitude and fourteen moments rounded to integers, per sample of the early
+# part that images reach the filter's 176 packed multiply-adds.
+FLOPS_PER_IMAGE = 150
+FLOPS_PER_SAMPLE = 4 * 176
 
 
 def _args():
@@ -606,32 +609,26 @@ def run_gpu(a):
         return
     updates, brute = workloads.windowed_updates(scene)
     ism_avg = sum(ism_ms) / len(ism_ms)
-    upd_per_s = updates / (ism_avg * 1e-3)
-    sfu_ach = upd_per_s * SFU_PER_UPDATE
-    fp32_ach = upd_per_s * FLOPS_PER_UPDATE
-    frac_sfu = sfu_ach / mufu_ops
-    frac_fp32 = fp32_ach / (fp32_flops / 2.0)
-    use_sfu = frac_sfu >= frac_fp32
+    images, samples = workloads.images_and_samples(scene)
+    fp32_ach = (images * FLOPS_PER_IMAGE + samples * FLOPS_PER_SAMPLE) / (ism_avg * 1e-3)
     traffic = _traffic(WORKLOAD)
     roofline = {
-        "bound": "sfu" if use_sfu else "fp32",
-        "achieved": (sfu_ach if use_sfu else fp32_ach) / 1e12,
-        "peak": (mufu_ops if use_sfu else fp32_flops / 2.0) / 1e12,
-        "unit": "Tops/s",
-        "frac": frac_sfu if use_sfu else frac_fp32,
+        "bound": "fp32",
+        "achieved": fp32_ach / 1e12,
+        "peak": fp32_flops / 1e12,
+        "unit": "TFLOP/s",
+        "frac": fp32_ach / fp32_flops,
         "traffic": traffic,
         "kernel": "ism_moment_kernel<256> (diffuse tail fused into its epilogue)",
-        "basis": "%d transcendental + %d FP32 ops per windowed image-sample update; %d updates "
-                 "per launch; peaks measured on this device (MUFU rcp, FP32 FMA)" %
-                 (SFU_PER_UPDATE, FLOPS_PER_UPDATE, updates),
-        "frac_fp32": frac_fp32, "frac_sfu": frac_sfu,
+        "basis": "%d FP32 operations per image in reach (%d) and %d per early sample that images reach (%d), "
+                 "as the kernel evaluates them; peak: FP32 FMA measured on this device" %
+                 (FLOPS_PER_IMAGE, images, FLOPS_PER_SAMPLE, samples),
         "peak_fp32_tflops_measured": fp32_flops / 1e12, "peak_mufu_tops_measured": mufu_ops / 1e12,
         "ism_ms": ism_avg,
         "why_not_hbm_or_tensor": "no contraction large enough for tensor cores and ~86 MB of DRAM "
-                                 "traffic per 0.3 ms launch: the kernel is bound by instruction issue and "
-                                 "shared-memory atomics, so its fraction is taken against the MUFU and FP32 "
-                                 "peaks measured on the device, over the operations of the reference formula "
-                                 "(above 1: the moments evaluate no window tap per image)",
+                                 "traffic per 0.3 ms launch: the kernel is bound by instruction issue (56 % of the "
+                                 "slots) and shared-memory atomics between its phases' barriers "
+                                 "(profiles/ism_moment.md)",
     }
     hbm_peak = _measured_hbm_gbs()
     if traffic and hbm_peak:

@@ -140,6 +140,28 @@ def windowed_updates(scene, chunk=1 << 22):
     return total, M * int(np.prod(nb)) * n_ism
 
 
+def images_and_samples(scene):
+    """Images of all pairs whose window reaches the early part, and the early samples up to the
+    last one that an image of the pair reaches."""
+    room, nb = np.asarray(scene["room_sz"], dtype=np.float64), np.asarray(scene["nb_img"], dtype=np.int64)
+    fs, c = float(np.float32(scene["fs"])), float(np.float32(scene.get("c", 343.0)))
+    n_ism = n_samples(scene.get("Tdiff") or scene["Tmax"], fs)
+    H = int(round(float(np.float32(8e-3) * np.float32(fs)))) / 2.0
+    pr = np.asarray(scene["pos_rcv"], dtype=np.float64)
+    images = samples = 0
+    for s in np.asarray(scene["pos_src"], dtype=np.float64):
+        v2 = []   # squared components per axis, [receivers, images of the axis]
+        for d in range(3):
+            k = np.arange(nb[d]) - nb[d] // 2
+            v = 2 * np.ceil(k / 2.0) * room[d] + (1 - 2 * np.abs(np.fmod(k, 2))) * s[d]
+            v2.append((v[None, :] - pr[:, d, None]) ** 2)
+        tau = np.sqrt(v2[0][:, :, None, None] + v2[1][:, None, :, None] + v2[2][:, None, None, :]) * (fs / c)
+        tau = tau.reshape(len(pr), -1)
+        images += int((tau < n_ism + H).sum())
+        samples += int(np.minimum(tau.max(axis=1) + H, n_ism).sum())
+    return images, samples
+
+
 def windowed_updates_torch(scene, device="cuda"):
     """windowed_updates computed with torch (FP64) on `device`, for large scenes."""
     import torch
