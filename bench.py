@@ -625,8 +625,8 @@ def run_gpu(a):
                  (FLOPS_PER_IMAGE, images, FLOPS_PER_SAMPLE, samples),
         "peak_fp32_tflops_measured": fp32_flops / 1e12, "peak_mufu_tops_measured": mufu_ops / 1e12,
         "ism_ms": ism_avg,
-        "why_not_hbm_or_tensor": "no contraction large enough for tensor cores and ~86 MB of DRAM "
-                                 "traffic per 0.3 ms launch: the kernel is bound by instruction issue (56 % of the "
+        "why_not_hbm_or_tensor": "no contraction large enough for tensor cores and ~77 MB of DRAM "
+                                 "traffic per 0.3 ms launch: the kernel is bound by instruction issue (58 % of the "
                                  "slots) and shared-memory atomics between its phases' barriers "
                                  "(profiles/ism_moment.md)",
     }

@@ -44,13 +44,13 @@
 // images than the integers hold is done again with bounds that fit.
 //
 // What bounds it: the shared-memory atomics of the image loop (2.7 cycles per warp at random
-// cells, 3.6 wavefronts; an FP32 atomicAdd takes 9.3 cycles) where images are many -- the
-// load pipe is at 77 % on 128 rooms -- and issue with the phases' barriers where they are few
-// (56 % of the slots on the array).  Per launch, ism_forward.cu and this kernel: one dense RIR of
+// cells, 3.5 wavefronts; an FP32 atomicAdd takes 9.3 cycles) where images are many -- the
+// load pipe is at 75 % on 128 rooms -- and issue with the phases' barriers where they are few
+// (58 % of the slots on the array).  Per launch, ism_forward.cu and this kernel: one dense RIR of
 // 6 million images 531 and 92 us, 64 x 32 array 490 and 321, 128 rooms 2680 and 642, 15 RIRs at
 // 48 kHz 87 and 37 (with one scale per segment 90, 321, 617 and 37).  (Other ways that were built first: a counting sort by cell with one
 // thread per cell adding in image order needed 8 barriers per 1024 images and ran at 228
-// cycles per 32 images and SM, against 90 here.)
+// cycles per 32 images and SM, against 93 here.)
 #include <algorithm>
 #include <cmath>
 #include <cstddef>
