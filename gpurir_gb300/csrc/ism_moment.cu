@@ -4,9 +4,9 @@
 // (src/gpuRIR_cuda.cu:110-121).  ism_forward.cu adds each image's Tw taps one by one;
 // this kernel separates them.  Time is cut into cells of two samples; with tau = n + u, n
 // the cell's centre and u in [-1, 1], each tap W(kappa - u), kappa = t - n, is a smooth
-// function of u and a polynomial of degree 13 reproduces all of them (3 to 4e-8 relative L2, 6e-8 at
-// the shortest windows; of the images whose window ends in the middle of a cell 5e-8 from 80 samples
-// of window on, up to 2.1e-7 below, all of it in the last tap):
+// function of u and a polynomial of degree 13 reproduces all of them (2 to 5e-8 relative L2, up to
+// 6.5e-8 at windows below 80 samples; of an image whose window ends in the middle of a cell at
+// most 7.3e-8, and 2.7e-7 below 80 samples, nearly all of it in the last tap):
 //   y[t] = sum over cells n, sum_j c_j(t - n) A_j[n],   A_j[n] = sum over the cell's images of a T_j(u)
 // with T_j the Chebyshev polynomials.  An image then costs its geometry and fourteen
 // multiply-adds instead of Tw taps, and a sample costs a fixed filter whatever the number
